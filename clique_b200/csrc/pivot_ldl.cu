@@ -11,9 +11,10 @@
 //
 // GPU form, per tree level after its extend-add and assembly, right-looking
 // in panels of 64 (65 when a 2 x 2 block closes the panel) columns:
-//   bk_panel_kernel   one CTA per front (1024 threads, 512 for FP64; on the
-//                     top levels a cluster of 8 CTAs per front): the panel's pivots one column at a
-//                     time.  The candidate columns are formed with the
+//   bk_panel_kernel   one CTA per front, or a cluster of 2 to 8 where a level
+//                     has few: the panel's pivots, 16 columns at a time while
+//                     no interchange is needed, else one column at a time.
+//                     The candidate columns are formed with the
 //                     panel's pending update (A(:,k) - L(:,panel) B(k,panel)^T,
 //                     B = D op(L)^T built from L and D on the fly), the pivot
 //                     search runs over the front's remaining pivot rows, a
@@ -63,10 +64,12 @@ namespace piv {
 
 constexpr int kNb = 64;                 // panel width (one more when a 2 x 2 block closes it)
 constexpr int kMaxPanel = kNb + 1;
-// threads of a panel CTA: as many loads in flight as the registers allow
-// (FP32: 51-62 registers a thread, 1024 threads; FP64: up to 126, 512)
-template <class T> constexpr int panel_threads() { return sizeof(T) == 4 ? 1024 : 512; }
-constexpr int kClusterCTAs = 8;         // CTAs sharing a front's panel on the top levels
+// row threads of a panel CTA (a block of speculative columns keeps kSpec
+// entries of a row in registers: FP32 up to 32 of them, FP64 up to 64), and
+// one more warp that factors the columns' diagonal block meanwhile
+template <class T> constexpr int panel_row_threads() { return sizeof(T) == 4 ? 512 : 256; }
+template <class T> constexpr int panel_threads() { return panel_row_threads<T>() + 32; }
+constexpr int kSpec = 16;               // columns taken at a time while no interchange is needed
 constexpr int kLowerRows = 128;         // rows of A21 per bk_lower_kernel CTA
 constexpr int kUpdThreads = 256;
 constexpr int kUpdTile = 64;
@@ -170,22 +173,100 @@ __device__ __forceinline__ void block_argmax(T& v, int& idx, T* sv, int* si) {
 }
 
 // ---------------------------------------------------------------------------
+// LDL^T without interchanges of the kSpec x kSpec (w used) block of a group
+// of speculative columns, by one warp: lane r (and r + 16) holds row r.  The
+// rows' pending update is sum_p L(r, p) B(c, p) over the panel's np factored
+// columns, the two half-warps taking alternate p.  Leaves L11 (unit lower, column
+// by column), the pivots and their reciprocals, and returns the first column
+// whose pivot fails the Bunch-Kaufman test against the block's own rows (or
+// whose reciprocal would leave the range); w when none does.
+// ---------------------------------------------------------------------------
+template <class T, bool C, bool CJ>
+__device__ __forceinline__ int spec_block(int np, int w, const V<T, C>* s_l, const V<T, C>* s_b, const V<T, C>* s_a,
+                                          V<T, C>* s_l11, V<T, C>* s_dn, V<T, C>* s_rd) {
+    using X = V<T, C>;
+    const int lane = threadIdx.x & 31, r = lane & (kSpec - 1), half = lane / kSpec;
+    X a[kSpec];
+#pragma unroll
+    for (int c = 0; c < kSpec; ++c) a[c] = (half == 0 && r < w && c <= r) ? s_a[c * kSpec + r] : X{};
+    for (int p = half; p < np; p += 2) {
+        const X l = neg(s_l[p * kSpec + r]);
+#pragma unroll
+        for (int c = 0; c < kSpec; ++c) mac(a[c], l, s_b[p * kSpec + c]);
+    }
+    auto shfl = [](X v, int src) -> X {
+        if constexpr (C) return X{__shfl_sync(0xffffffffu, v.r, src), __shfl_sync(0xffffffffu, v.i, src)};
+        else return __shfl_sync(0xffffffffu, v, src);
+    };
+#pragma unroll
+    for (int c = 0; c < kSpec; ++c) a[c] += shfl(a[c], lane ^ kSpec);
+    int fail = w;
+#pragma unroll
+    for (int j = 0; j < kSpec; ++j) {
+        if (j < w) {
+            X d = shfl(a[j], j);
+            if constexpr (CJ) d = realpart(d);
+            const T md = mag1(d);
+            const bool zero = md == T(0);
+            const T lo = sizeof(T) == 4 ? T(1e-30) : T(1e-290), hi = sizeof(T) == 4 ? T(1e30) : T(1e290);
+            const bool bad = r > j && r < w && !(md >= (T)kAlpha * mag1(a[j]));
+            if (__ballot_sync(0xffffffffu, bad || !(zero || (md > lo && md < hi)))) fail = min(fail, j);
+            const X rd = zero ? X{} : vone<X>() / d;
+            const X l = a[j] * rd;
+            if (lane == 0) {
+                s_dn[j] = d;
+                s_rd[j] = rd;
+            }
+            if (half == 0) s_l11[j * kSpec + r] = r > j ? l : X{};
+#pragma unroll
+            for (int c = j + 1; c < kSpec; ++c) {
+                const X b = opc<CJ>(shfl(a[j], c));
+                mac(a[c], neg(l), b);   // (used for r >= c only)
+            }
+        }
+    }
+    return fail;
+}
+
+// ---------------------------------------------------------------------------
 // one panel of Bunch-Kaufman pivots per front: one CTA (G = 1), or a
-// cluster of G CTAs sharing the front's rows (the top levels, whose few
-// large fronts would leave most SMs idle).  With G > 1 every CTA takes the
-// rows k + rank nt + tid + q G nt, the argmax partials meet in the first
-// CTA's shared memory, every CTA reaches the same pivot decisions from the
-// same combined values (so all pass the same cluster barriers), the entries
-// other CTAs wrote are read from L2 (ld.global.cg), and the first CTA's
-// thread 0 does the single-entry work
+// cluster of G CTAs sharing the front's rows (levels of few large fronts,
+// which would leave most SMs idle).  Every CTA of a cluster reaches the same
+// pivot decisions from the same combined values (so all pass the same
+// cluster barriers), the entries other CTAs wrote are read from L2
+// (ld.global.cg), and the first CTA's thread 0 does the single-entry work.
+//
+// Columns are taken kSpec at a time as long as Bunch-Kaufman would choose the
+// diagonal entry without an interchange, |a_kk| >= alpha max_i |a_ik|, in
+// every one of them: no interchange means that the columns are those of the
+// unpivoted elimination, so the group is eliminated without a search (its
+// diagonal block by one warp of every CTA, the rows below it one a thread,
+// with the group's kSpec entries in registers) and each row tests its own
+// entries against the pivots.  The first column in which any row fails ends
+// the accepted prefix (the maximum over rows passes exactly when every row
+// does), nothing of the later columns has been written, and that column goes
+// through the general step below: candidate column and, where needed, row,
+// search, interchange, 1 x 1 or 2 x 2 pivot.  What bounds the general step is
+// its chain of L2 round trips and cluster barriers, 8.4 us a column with
+// 8 CTAs; a group of 16 columns passes two barriers.  Pivoted factor + refined
+// solve of 48^3 Helmholtz, CFP32: 56.3 -> 21.4 ms (panels were 41 ms of it);
+// indefinite operators, FP64: Hermitian 40 x 37 x 33 (1929 interchanged rows
+// in 48840) 28.4 -> 22.3 ms, real 29 x 27 x 23 in graph order 6.8 -> 5.2 ms.
 // ---------------------------------------------------------------------------
 template <class T, bool C, bool CJ, int G = 1>
 __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
                                                                  T* __restrict__ L, double* __restrict__ D, double* __restrict__ E,
                                                                  int32_t* __restrict__ pivg, T* __restrict__ cvec, T* __restrict__ vvec,
-                                                                 int32_t* __restrict__ state, int32_t* __restrict__ status) {
+                                                                 int32_t* __restrict__ state, int32_t* __restrict__ status,
+                                                                 int wspec) {
     using X = V<T, C>;
     using W = DV<C>;
+    extern __shared__ __align__(16) unsigned char bk_panel_smem[];
+    X* s_y = reinterpret_cast<X*>(bk_panel_smem);   // speculative columns: entry c of row slot q at c * slots + q
+    __shared__ X s_gl[kNb * kSpec], s_gb[kNb * kSpec];   // the group's rows of the factored columns, and B of them
+    __shared__ X s_ga[kSpec * kSpec], s_gl11[kSpec * kSpec], s_gd[kSpec], s_grd[kSpec];
+    __shared__ int s_fail;
+    __shared__ int s_slot_f[G];
     __shared__ X s_d[kMaxPanel], s_e[kMaxPanel];   // the panel's D (diagonal, and D(p+1,p) of 2 x 2 blocks)
     __shared__ X s_w[kMaxPanel];                   // B(k, p)
     __shared__ X s_lr[kMaxPanel], s_wi[kMaxPanel]; // L(imax, p), B(imax, p)
@@ -227,9 +308,117 @@ __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const Fron
     if (j0 == 0)
         for (int i = t0; i < n; i += ntot) pivg[f.off + i] = f.off + i;
     const int jend = min(n, j0 + kNb);
+    const int rt = nt - 32, slots = ((n + G * rt - 1) / (G * rt)) * rt;   // row threads, row slots of this CTA
+    bool general = false;
+    if constexpr (G > 1) cg::this_cluster().sync();   // every CTA's shared memory is there
     int k = j0;
     while (k < jend) {
         const int np = k - j0;
+        const int w = min(wspec, jend - k);
+        if (w > 1 && !general) {
+            for (int idx = tid; idx < np * kSpec; idx += nt) {
+                const int r = idx % kSpec, p = idx / kSpec;
+                s_gl[idx] = r < w ? ld(L, at(k + r, j0 + p)) : X{};
+            }
+            for (int idx = tid; idx < kSpec * kSpec; idx += nt) {
+                const int r = idx % kSpec, c = idx / kSpec;
+                s_ga[idx] = (r < w && c <= r) ? ld(L, at(k + r, k + c)) : X{};
+            }
+            if (tid == 0) s_fail = w;
+            __syncthreads();
+            for (int idx = tid; idx < np * kSpec; idx += nt) {
+                const int c = idx % kSpec, p = idx / kSpec;
+                s_gb[idx] = bval<CJ>(p, s_d[p], s_e[p], p > 0 ? s_e[p - 1] : X{}, p > 0,
+                                     [&](int q) { return s_gl[q * kSpec + c]; });
+            }
+            __syncthreads();
+            const int i0 = k + w;
+            if (tid >= rt) {   // the last warp
+                const int f0 = spec_block<T, C, CJ>(np, w, s_gl, s_gb, s_ga, s_gl11, s_gd, s_grd);
+                if (tid == rt) atomicMin(&s_fail, f0);
+                __syncthreads();
+            } else {
+                int fail = w;
+                for (int q = 0; q == 0 || q * rt < slots; ++q) {
+                    const int i = i0 + rank * rt + tid + q * G * rt;
+                    const bool in = i < n;
+                    X y[kSpec];
+#pragma unroll
+                    for (int c = 0; c < kSpec; ++c) y[c] = (in && c < w) ? ld(L, at(i, k + c)) : X{};
+                    if (in) {
+                        constexpr int kFly = C && sizeof(T) == 8 ? 4 : 8;   // loads in flight
+                        int p = 0;
+                        for (; p + kFly <= np; p += kFly) {
+                            X l[kFly];
+#pragma unroll
+                            for (int t = 0; t < kFly; ++t) l[t] = ld(L, at(i, j0 + p + t));
+#pragma unroll
+                            for (int t = 0; t < kFly; ++t) {
+                                const X nl = neg(l[t]);
+#pragma unroll
+                                for (int c = 0; c < kSpec; ++c) mac(y[c], nl, s_gb[(p + t) * kSpec + c]);
+                            }
+                        }
+                        for (; p < np; ++p) {
+                            const X nl = neg(ld(L, at(i, j0 + p)));
+#pragma unroll
+                            for (int c = 0; c < kSpec; ++c) mac(y[c], nl, s_gb[p * kSpec + c]);
+                        }
+                    }
+                    if (q == 0) __syncthreads();   // the block's factors are there
+                    if (in) {
+#pragma unroll
+                        for (int c = 0; c < kSpec; ++c) {
+                            if (c < w) {
+                                if (!(mag1(s_gd[c]) >= (T)kAlpha * mag1(y[c]))) fail = min(fail, c);
+                                s_y[c * slots + q * rt + tid] = y[c] * s_grd[c];
+                                const X ny = neg(y[c]);
+#pragma unroll
+                                for (int t = c + 1; t < kSpec; ++t) mac(y[t], ny, opc<CJ>(s_gl11[c * kSpec + t]));
+                            }
+                        }
+                    }
+                }
+                fail = __reduce_min_sync(0xffffffffu, fail);
+                if ((tid & 31) == 0 && fail < w) atomicMin(&s_fail, fail);
+            }
+            __syncthreads();
+            int kf = s_fail;
+            if constexpr (G > 1) {
+                if (tid < G) cg::this_cluster().map_shared_rank(s_slot_f, tid)[rank] = kf;
+                sync();
+#pragma unroll
+                for (int q = 0; q < G; ++q) kf = min(kf, s_slot_f[q]);
+            }
+            // the accepted columns
+            if (tid < rt) {
+                for (int q = 0; q * rt < slots; ++q) {
+                    const int i = i0 + rank * rt + tid + q * G * rt;
+                    if (i >= n) break;
+                    for (int c = 0; c < kf; ++c) stv<T, C>(L, at(i, k + c), s_y[c * slots + q * rt + tid]);
+                }
+            }
+            if (rank == 0) {
+                for (int idx = tid; idx < kSpec * kf; idx += nt) {
+                    const int r = idx % kSpec, c = idx / kSpec;
+                    if (r < w && r >= c) stv<T, C>(L, at(k + r, k + c), r == c ? vone<X>() : s_gl11[idx]);
+                }
+                if (tid < kf) {
+                    reinterpret_cast<W*>(D)[f.off + k + tid] = conv<W>(s_gd[tid]);
+                    reinterpret_cast<W*>(E)[f.off + k + tid] = W{};
+                    if (is_zero(s_gd[tid])) atomicMin(&status[0], __ldcg(pivg + f.off + k + tid) + 1);
+                }
+            }
+            if (tid < kf) {
+                s_d[np + tid] = s_gd[tid];
+                s_e[np + tid] = X{};
+            }
+            sync();
+            k += kf;
+            general = kf < w;
+            continue;
+        }
+        general = false;
         // B(k, p) for the panel's factored columns
         if (tid < np) {
             const int p = j0 + tid;
@@ -867,6 +1056,74 @@ __global__ void quasi_diag_kernel(T* __restrict__ X, int64_t ldx, int64_t n, int
     }
 }
 
+// launch shape of a level's panels: CTAs a front, row threads a CTA, columns
+// taken speculatively at a time and the shared memory of their rows
+struct PanelShape {
+    int ctas, rows, wspec;
+    size_t smem;
+};
+
+constexpr size_t kPanelDynSmem = 160 * 1024;   // beside up to 48 KB of static shared memory
+
+template <class T>
+static PanelShape panel_shape(int64_t nfronts, int max_n, int elem) {
+    PanelShape s{};
+    s.rows = max_n <= 128 ? 128 : max_n <= 256 ? 256 : panel_row_threads<T>();
+    auto fits = [&](int w) {
+        const int64_t slots = (max_n + (int64_t)s.ctas * s.rows - 1) / ((int64_t)s.ctas * s.rows) * s.rows;
+        s.wspec = w;
+        s.smem = (size_t)(slots * w * elem);
+        return s.smem <= kPanelDynSmem;
+    };
+    s.ctas = 1;
+    while (s.ctas < 8 && nfronts * s.ctas * 2 <= 148 && max_n > s.ctas * 128) s.ctas *= 2;
+    if (fits(kSpec)) return s;
+    s.ctas = 8;   // too many rows for the shared memory of fewer CTAs
+    for (int w = kSpec; w > 1; w /= 2)
+        if (fits(w)) return s;
+    s.wspec = 0;
+    s.smem = 0;
+    return s;
+}
+
+template <class T, bool C, bool CJ, int G>
+static bool launch_panel_g(Plan& P, const int32_t* fl, int nfronts, const PanelShape& sh, T* L, T* cvec, T* vvec, cudaStream_t st) {
+    static const bool attr = cudaFuncSetAttribute(bk_panel_kernel<T, C, CJ, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)kPanelDynSmem) == cudaSuccess;
+    if (!attr) return false;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nfronts * G));
+    cfg.blockDim = dim3((unsigned)(sh.rows + 32));
+    cfg.dynamicSmemBytes = sh.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = G;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = G > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, bk_panel_kernel<T, C, CJ, G>, (const FrontDev*)P.fronts, fl, L, P.D, P.E, P.pivg, cvec,
+                                       vvec, P.pstate, P.status, sh.wspec) == cudaSuccess;
+}
+
+template <class T, bool C, bool CJ>
+static int launch_panel(Plan& P, const int32_t* fl, int nfronts, const PanelShape& sh, T* L, T* cvec, T* vvec, cudaStream_t st) {
+    bool done = false;
+    if (sh.ctas == 8) done = launch_panel_g<T, C, CJ, 8>(P, fl, nfronts, sh, L, cvec, vvec, st);
+    if (sh.ctas == 4) done = launch_panel_g<T, C, CJ, 4>(P, fl, nfronts, sh, L, cvec, vvec, st);
+    if (sh.ctas == 2) done = launch_panel_g<T, C, CJ, 2>(P, fl, nfronts, sh, L, cvec, vvec, st);
+    if (done) return CLIQ_OK;
+    PanelShape one = sh;
+    if (sh.ctas > 1) {   // one CTA a front takes its columns one by one
+        cudaGetLastError();
+        one.ctas = 1;
+        one.wspec = 0;
+        one.smem = 0;
+    }
+    return launch_panel_g<T, C, CJ, 1>(P, fl, nfronts, one, L, cvec, vvec, st) ? CLIQ_OK : check_cuda("pivoted panel");
+}
+
 template <class T, bool C, bool CJ>
 static int level_t(Plan& P, int depth, cudaStream_t st, bool schur) {
     const SolveLevel& lv = P.solve_levels[depth];
@@ -901,37 +1158,13 @@ static int level_t(Plan& P, int depth, cudaStream_t st, bool schur) {
     const bool wide = std::is_same<T, float>::value && !tile64;
     // FP64: the in-front updates on DMMA where the plan's FP64 updates are
     const bool dmma_front = std::is_same<T, double>::value && P.fp64_dmma && !tile64;
-    // the top levels (a few large fronts): each front's panels on a cluster
-    // of kClusterCTAs CTAs; a refused cluster launch falls back to one CTA a front
-    const bool clustered = (int64_t)lv.nfronts * kClusterCTAs <= 148 && max_n >= 512;
-    // one CTA a front otherwise; a column step works over the front's pivot
-    // rows only, so fronts of at most 128 / 256 pivots take CTAs of that many
-    // threads (several CTAs a SM on the deep levels' many small fronts; at
-    // least kMaxPanel threads, which the panel's per-column loads need)
-    const int narrow = max_n <= 128 ? 128 : max_n <= 256 ? 256 : panel_threads<T>();
-    static_assert(kMaxPanel <= 128, "panel CTAs of 128 threads");
+    // CTAs a front's panel is shared by: as many as the level's fronts leave
+    // room for on the 148 SMs (fronts of at most a CTA's worth of rows gain
+    // nothing from more), at least what the speculative columns' rows need in
+    // shared memory; a refused cluster launch falls back to one CTA a front
+    const PanelShape shape = panel_shape<T>(lv.nfronts, max_n, (int)sizeof(V<T, C>));
     for (int step = 0; step < steps; ++step) {
-        bool done = false;
-        if (clustered) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(lv.nfronts * kClusterCTAs));
-            cfg.blockDim = dim3(panel_threads<T>());
-            cfg.dynamicSmemBytes = 0;
-            cfg.stream = st;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = kClusterCTAs;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            done = cudaLaunchKernelEx(&cfg, bk_panel_kernel<T, C, CJ, kClusterCTAs>, (const FrontDev*)P.fronts, fl, L, P.D, P.E,
-                                      P.pivg, cvec, vvec, P.pstate, P.status) == cudaSuccess;
-            if (!done) cudaGetLastError();
-        }
-        if (!done)
-            bk_panel_kernel<T, C, CJ><<<(unsigned)lv.nfronts, narrow, 0, st>>>(P.fronts, fl, L, P.D, P.E, P.pivg, cvec, vvec,
-                                                                           P.pstate, P.status);
+        TRY((launch_panel<T, C, CJ>(P, fl, lv.nfronts, shape, L, cvec, vvec, st)));
         if (max_u > 0)
             bk_lower_kernel<T, C, CJ><<<(unsigned)((int64_t)lv.nfronts * chunks), kLowerRows, smem_lower, st>>>(
                 P.fronts, fl, chunks, L, P.D, P.E, P.pstate);

@@ -372,3 +372,44 @@ def test_intrapiv_fp64_in_front_update_on_dmma(kind, monkeypatch):
     # measured: 0 (real: both kernels sum each entry's products as fused
     # multiply-adds in k order), 7.0e-16 (complex), 6.1e-12 (Hermitian)
     assert worst <= 1e-10
+
+
+@pytest.mark.parametrize("kind", ["real", "complex", "hermitian"])
+@pytest.mark.parametrize("dims", [(15, 1, 1), (16, 1, 1), (17, 1, 1), (13, 5, 1), (16, 8, 1), (43, 3, 1), (16, 16, 1),
+                                  (257, 1, 1), (19, 9, 3)])
+@pytest.mark.parametrize("weak", [0, 1, 37])
+def test_intrapiv_speculative_columns(oracle, kind, dims, weak):
+    """One front of 15 .. 513 pivots (one to eight CTAs a panel), no column,
+    one column in the middle or every 37th one with a small diagonal: groups
+    of columns taken without a search end at any offset.  Pivot order and 2x2
+    blocks as the oracle's; L and D to 1e-10 of the front's largest entry, as
+    the other pivoted fronts."""
+    base = ops.laplacian_3d(*dims, 6.5)
+    vals = base.values.astype(np.complex128 if kind != "real" else np.float64)
+    rows = np.repeat(np.arange(base.n), np.diff(base.rowptr))
+    off = base.colind != rows
+    if kind == "hermitian":
+        vals[off] = vals[off] * np.exp(1j * 0.4 * np.sign(base.colind - rows))[off]
+    if kind == "complex":
+        vals[~off] = vals[~off] * (1 + 0.2j)
+    small = rows % 37 == 5 if weak == 37 else rows == base.n // 2 if weak else np.zeros(len(rows), bool)
+    vals[small & ~off] *= 0.01
+    A = _perturbed(base, vals)
+    conj = kind == "hermitian"
+    n = A.n
+    _, _, L = _tree(A, dims, n, "double", conj)
+    S = oracle.Symbolic(*dims, A.rowptr, A.colind, cutoff=n)
+    F = oracle.Fronts(S, A.values, is_complex=kind != "real", conjugate=conj)
+    assert F.ldl(96, pivot=True) == 0
+    assert S.num_nodes == 1
+    Lo, do = F.front(0)
+    so, po = F.pivots(0)
+    Lg, dg = L.front(0)
+    sg, pg = L.front_pivots(0)
+    assert np.array_equal(pg, po)
+    assert np.array_equal(sg != 0, so != 0)
+    if weak:
+        assert (po != np.arange(n)).any() or (so != 0).any()
+    scale = max(np.abs(Lo).max(), np.abs(do).max())
+    for g, o in ((Lg, Lo), (dg, do), (sg, so)):
+        assert np.abs(g - o).max() <= 1e-10 * scale
