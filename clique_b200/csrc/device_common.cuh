@@ -70,6 +70,49 @@ template <class T> __device__ __forceinline__ void mac(cx<T>& acc, cx<T> a, cx<T
     acc.i = fma(a.r, b.i, acc.i); acc.i = fma(a.i, b.r, acc.i);
 }
 
+// Reciprocal of a pivot, on the critical path of every elimination step.
+// 1/x for x within float range: Newton-Raphson iteration y <- y (2 - x y)
+// from the single-precision reciprocal (about 23 correct bits, two steps
+// give full double precision); outside that range the IEEE reciprocal.
+// Complex: conj(d) / |d|^2, with d scaled by a power of two when |d|^2
+// would leave the range.
+__device__ __forceinline__ double recip_nr(double x) {
+    const double ax = fabs(x);
+    if (!(ax > 1e-30 && ax < 1e30)) return __drcp_rn(x);
+    double y = (double)__frcp_rn((float)x);
+    y = y * fma(-x, y, 2.0);
+    y = y * fma(-x, y, 2.0);
+    return y;
+}
+__device__ __forceinline__ float pivot_recip(float d) { return __frcp_rn(d); }
+__device__ __forceinline__ cx<float> pivot_recip(cx<float> d) {
+    const float n2 = fmaf(d.r, d.r, d.i * d.i);
+    if (n2 > 1e-36f && n2 < 1e36f) {
+        const float s = __frcp_rn(n2);
+        return {d.r * s, -d.i * s};
+    }
+    const float mx = fmaxf(fabsf(d.r), fabsf(d.i));
+    const int e = ((__float_as_int(mx) >> 23) & 0xff) - 127;
+    const float sc = __int_as_float((127 - e) << 23);   // 2^-e
+    const float xr = d.r * sc, xi = d.i * sc;
+    const float s = __frcp_rn(fmaf(xr, xr, xi * xi)) * sc;
+    return {xr * s, -xi * s};
+}
+__device__ __forceinline__ double pivot_recip(double d) { return recip_nr(d); }
+__device__ __forceinline__ cx<double> pivot_recip(cx<double> d) {
+    const double n2 = fma(d.r, d.r, d.i * d.i);
+    if (n2 > 1e-30 && n2 < 1e30) {
+        const double s = recip_nr(n2);
+        return {d.r * s, -d.i * s};
+    }
+    const double mx = fmax(fabs(d.r), fabs(d.i));
+    const int e = ((__double2hiint(mx) >> 20) & 0x7ff) - 1023;
+    const double sc = __hiloint2double((1023 - e) << 20, 0);   // 2^-e
+    const double xr = d.r * sc, xi = d.i * sc;
+    const double s = __drcp_rn(fma(xr, xr, xi * xi)) * sc;
+    return {xr * s, -xi * s};
+}
+
 // element load / store from a T* arena
 template <class T, bool C> __device__ __forceinline__ V<T, C> ldv(const T* p, int64_t e) {
     return reinterpret_cast<const V<T, C>*>(p)[e];

@@ -142,49 +142,6 @@ __host__ __device__ constexpr size_t diag_smem_bytes() {
     return sizeof(DiagW<WT, C>) * (size_t)(kTile * kDiagLd + kTile * kSub + 4 * kSub * kSubLd + 2 * kTile);
 }
 
-// Reciprocal of a pivot, on the critical path of every elimination step.
-// 1/x for x within float range: Newton-Raphson iteration y <- y (2 - x y)
-// from the single-precision reciprocal (about 23 correct bits, two steps
-// give full double precision); outside that range the IEEE reciprocal.
-// Complex: conj(d) / |d|^2, with d scaled by a power of two when |d|^2
-// would leave the range.
-__device__ __forceinline__ double recip_nr(double x) {
-    const double ax = fabs(x);
-    if (!(ax > 1e-30 && ax < 1e30)) return __drcp_rn(x);
-    double y = (double)__frcp_rn((float)x);
-    y = y * fma(-x, y, 2.0);
-    y = y * fma(-x, y, 2.0);
-    return y;
-}
-__device__ __forceinline__ float pivot_recip(float d) { return __frcp_rn(d); }
-__device__ __forceinline__ cx<float> pivot_recip(cx<float> d) {
-    const float n2 = fmaf(d.r, d.r, d.i * d.i);
-    if (n2 > 1e-36f && n2 < 1e36f) {
-        const float s = __frcp_rn(n2);
-        return {d.r * s, -d.i * s};
-    }
-    const float mx = fmaxf(fabsf(d.r), fabsf(d.i));
-    const int e = ((__float_as_int(mx) >> 23) & 0xff) - 127;
-    const float sc = __int_as_float((127 - e) << 23);   // 2^-e
-    const float xr = d.r * sc, xi = d.i * sc;
-    const float s = __frcp_rn(fmaf(xr, xr, xi * xi)) * sc;
-    return {xr * s, -xi * s};
-}
-__device__ __forceinline__ double pivot_recip(double d) { return recip_nr(d); }
-__device__ __forceinline__ cx<double> pivot_recip(cx<double> d) {
-    const double n2 = fma(d.r, d.r, d.i * d.i);
-    if (n2 > 1e-30 && n2 < 1e30) {
-        const double s = recip_nr(n2);
-        return {d.r * s, -d.i * s};
-    }
-    const double mx = fmax(fabs(d.r), fabs(d.i));
-    const int e = ((__double2hiint(mx) >> 20) & 0x7ff) - 1023;
-    const double sc = __hiloint2double((1023 - e) << 20, 0);   // 2^-e
-    const double xr = d.r * sc, xi = d.i * sc;
-    const double s = __drcp_rn(fma(xr, xr, xi * xi)) * sc;
-    return {xr * s, -xi * s};
-}
-
 template <class T, bool C, bool CJ, class WT>
 __global__ void __launch_bounds__(kThreads, 2) diag_ldl_kernel(const FrontDev* __restrict__ F, const int4* __restrict__ items, int k,
                                                                T* __restrict__ L, double* __restrict__ D, T* __restrict__ tinv,
@@ -850,7 +807,6 @@ static int issue_factor_pivoted(Plan& P, int64_t* nlaunch) {
         const bool on_tc = tc_ok[ln.depth] != 0;
         TRY(pivot_level(P, ln.depth, st, !on_tc));
         if (on_tc && !schur[ln.depth].empty()) {
-            if (std::is_same<T, float>::value) TRY(pivot_rowmax(P, ln.depth, st));
             for (size_t li : schur[ln.depth]) {
                 if (std::is_same<T, float>::value) launch_tc2(P, P.launches[li], nullptr, st, P.pack);
                 else launch_dmma_update(P, P.launches[li], st);

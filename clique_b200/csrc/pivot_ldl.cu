@@ -32,7 +32,7 @@
 //                     panel state), bk_update_kernel without DMMA.
 // At the end of the level the Schur complements (K = n) go into the update
 // pool through the plan's own Schur launches -- tcgen05 for FP32 plans
-// (bk_rowmax_kernel gives the 2xFP16 split's row maxima; the packing's
+// (bk_lower_kernel gives the 2xFP16 split's row maxima; the packing's
 // pivoted variant forms S = D op(L) with the 2 x 2 terms), DMMA for FP64
 // plans (halo rows for the 2 x 2 terms) -- or through bk_update_kernel.
 // Then the 64 x 64 diagonal-block inverses the sweeps use, and the index
@@ -49,6 +49,7 @@
 #include <string>
 
 #include <cooperative_groups.h>
+#include <cuda_pipeline.h>
 namespace cg = cooperative_groups;
 
 #ifndef TRY
@@ -211,7 +212,9 @@ __device__ __forceinline__ int spec_block(int np, int w, const V<T, C>* s_l, con
             const T lo = sizeof(T) == 4 ? T(1e-30) : T(1e-290), hi = sizeof(T) == 4 ? T(1e30) : T(1e290);
             const bool bad = r > j && r < w && !(md >= (T)kAlpha * mag1(a[j]));
             if (__ballot_sync(0xffffffffu, bad || !(zero || (md > lo && md < hi)))) fail = min(fail, j);
-            const X rd = zero ? X{} : vone<X>() / d;
+            X rd{};
+            if constexpr (CJ) rd.r = zero ? T(0) : T(1) / d.r;
+            else rd = zero ? X{} : pivot_recip(d);
             const X l = a[j] * rd;
             if (lane == 0) {
                 s_dn[j] = d;
@@ -596,17 +599,25 @@ __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const Fron
 }
 
 // ---------------------------------------------------------------------------
-// rows below the pivots: L21(:, panel) = A21(:, panel) op(L11)^{-T} D^{-1}
+// rows below the pivots: L21(:, panel) = A21(:, panel) op(L11)^{-T} D^{-1},
+// one row a thread.  The row's panel entries are all fetched at once into
+// shared memory (asynchronous copies, beside the loads of L11), then
+// substituted kSpec columns at a time with the group's entries in registers:
+// one entry of y = L21 D read back feeds kSpec products.  What bounds a
+// launch is that chain for one row.  For the 2xFP16 split of the Schur
+// complements the row's largest |component| of L21 and of y (which |B| is)
+// goes into the two halves of erow (float bits), panel after panel.
 // ---------------------------------------------------------------------------
 template <class T, bool C, bool CJ>
 __global__ void __launch_bounds__(kLowerRows) bk_lower_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl, int chunks,
                                                               T* __restrict__ L, const double* __restrict__ D,
-                                                              const double* __restrict__ E, const int32_t* __restrict__ state) {
+                                                              const double* __restrict__ E, const int32_t* __restrict__ state,
+                                                              uint32_t* __restrict__ erow, int64_t erow_total) {
     using X = V<T, C>;
     using W = DV<C>;
     extern __shared__ __align__(16) unsigned char bk_smem[];
-    X* s_l = reinterpret_cast<X*>(bk_smem);   // L11 of the panel, kMaxPanel x kMaxPanel, column-major, then the rows' y
-    __shared__ X s_d[kMaxPanel], s_e[kMaxPanel];
+    X* s_l = reinterpret_cast<X*>(bk_smem);   // L11 of the panel, kMaxPanel x kMaxPanel, column-major, then the rows' entries
+    __shared__ X s_d[kMaxPanel], s_e[kMaxPanel], s_rd[kMaxPanel];
     const int fi = blockIdx.x / chunks, ch = blockIdx.x % chunks;
     const int s = fl[fi];
     const FrontDev f = F[s];
@@ -614,41 +625,86 @@ __global__ void __launch_bounds__(kLowerRows) bk_lower_kernel(const FrontDev* __
     const int u = f.m - f.n;
     if (kb <= 0 || ch * kLowerRows >= u) return;
     const int64_t base = f.L;
-    for (int idx = threadIdx.x; idx < kb * kb; idx += blockDim.x) {
+    const int i = f.n + ch * kLowerRows + threadIdx.x;
+    const bool in = i < f.m;
+    const int64_t row = base + i + (int64_t)j0 * f.m;
+    X* y = s_l + kMaxPanel * kMaxPanel + threadIdx.x;   // this row's entry of column q at q * kLowerRows
+    if (in)
+        for (int q = 0; q < kb; ++q)
+            __pipeline_memcpy_async(y + q * kLowerRows, reinterpret_cast<const X*>(L) + row + (int64_t)q * f.m, sizeof(X));
+    __pipeline_commit();
+#pragma unroll 8
+    for (int idx = threadIdx.x; idx < kb * kb; idx += kLowerRows) {
         const int r = idx % kb, c = idx / kb;
         s_l[r + c * kMaxPanel] = r > c ? ldv<T, C>(L, base + (j0 + r) + (int64_t)(j0 + c) * f.m) : X{};
     }
-    for (int q = threadIdx.x; q < kb; q += blockDim.x) {
+    for (int q = threadIdx.x; q < kb; q += kLowerRows) {
         s_d[q] = conv<X>(reinterpret_cast<const W*>(D)[f.off + j0 + q]);
         s_e[q] = conv<X>(reinterpret_cast<const W*>(E)[f.off + j0 + q]);
+        // complex symmetric: reciprocals of the 1 x 1 pivots (a complex division
+        // is a few real ones in a row); 0 leaves an entry to the division (real
+        // pivots, pivots near the ends of the range)
+        const T md = mag1(s_d[q]);
+        const bool ok = C && !CJ && md > (sizeof(T) == 4 ? T(1e-30) : T(1e-290)) && md < (sizeof(T) == 4 ? T(1e30) : T(1e290));
+        s_rd[q] = ok ? pivot_recip(s_d[q]) : X{};
     }
+    __pipeline_wait_prior(0);   // (a thread reads back only the row it fetched)
     __syncthreads();
-    const int i = f.n + ch * kLowerRows + threadIdx.x;
-    if (i >= f.m) return;
-    const int64_t row = base + i;
-    // this thread's row of the panel in shared memory (column q at q * kLowerRows + tid): all loads first
-    X* y = s_l + kMaxPanel * kMaxPanel + threadIdx.x;
-    for (int q = 0; q < kb; ++q) y[q * kLowerRows] = ldv<T, C>(L, row + (int64_t)(j0 + q) * f.m);
+    if (!in) return;
     // y(q) = a(q) - sum_{p<q} y(p) op(L11(q, p))
-    for (int q = 1; q < kb; ++q) {
-        X a = y[q * kLowerRows];
-        for (int p = 0; p < q; ++p) a -= y[p * kLowerRows] * opc<CJ>(s_l[q + p * kMaxPanel]);
-        y[q * kLowerRows] = a;
+    for (int c0 = 0; c0 < kb; c0 += kSpec) {
+        const int w = min(kSpec, kb - c0);
+        X a[kSpec];
+#pragma unroll
+        for (int c = 0; c < kSpec; ++c) a[c] = c < w ? y[(c0 + c) * kLowerRows] : X{};
+        for (int p = 0; p < c0; ++p) {
+            const X ny = neg(y[p * kLowerRows]);
+            const X* l = s_l + c0 + p * kMaxPanel;   // (w < kSpec: reads on into the next column, not used)
+#pragma unroll
+            for (int c = 0; c < kSpec; ++c) mac(a[c], ny, opc<CJ>(l[c]));
+        }
+#pragma unroll
+        for (int c = 0; c < kSpec; ++c) {
+            if (c < w) {
+                const X ny = neg(a[c]);
+                const X* l = s_l + c0 + (c0 + c) * kMaxPanel;
+#pragma unroll
+                for (int t = c + 1; t < kSpec; ++t) mac(a[t], ny, opc<CJ>(l[t]));
+                y[(c0 + c) * kLowerRows] = a[c];
+            }
+        }
     }
     // l = y D^{-1}
+    auto big = [](X v) -> float {
+        if constexpr (C) return fmaxf(fabsf((float)v.r), fabsf((float)v.i));
+        else return fabsf((float)v);
+    };
+    float ml = 0.f, ms = 0.f;
+#pragma unroll 4
     for (int q = 0; q < kb; ++q) {
-        const int64_t e0 = row + (int64_t)(j0 + q) * f.m;
-        if (!is_zero(s_e[q])) {
-            const X d11 = s_d[q], d22 = s_d[q + 1], d21 = s_e[q];
-            const X det = d11 * d22 - d21 * opc<CJ>(d21);
-            const X y0 = y[q * kLowerRows], y1 = y[(q + 1) * kLowerRows];
-            stv<T, C>(L, e0, (y0 * d22 - y1 * d21) / det);
-            stv<T, C>(L, e0 + f.m, (y1 * d11 - y0 * opc<CJ>(d21)) / det);
-            ++q;
+        const X d = s_d[q], d21 = s_e[q], rd = s_rd[q], y0 = y[q * kLowerRows];
+        ms = fmaxf(ms, big(y0));
+        X l;
+        if (!is_zero(d21)) {
+            const X d22 = s_d[q + 1];
+            l = (y0 * d22 - y[(q + 1) * kLowerRows] * d21) / (d * d22 - d21 * opc<CJ>(d21));
+        } else if (q > 0 && !is_zero(s_e[q - 1])) {
+            const X d11 = s_d[q - 1], e = s_e[q - 1];
+            l = (y0 * d11 - y[(q - 1) * kLowerRows] * opc<CJ>(e)) / (d11 * d - e * opc<CJ>(e));
         } else {
-            const X d = s_d[q];
-            stv<T, C>(L, e0, is_zero(d) ? X{} : y[q * kLowerRows] / d);
+            if constexpr (CJ) l = d.r == T(0) ? X{} : X{y0.r / d.r, y0.i / d.r};
+            else l = !is_zero(rd) ? y0 * rd : is_zero(d) ? X{} : y0 / d;
         }
+        ml = fmaxf(ml, big(l));
+        stv<T, C>(L, row + (int64_t)q * f.m, l);
+    }
+    if (erow) {
+        if (j0 > 0) {
+            ml = fmaxf(ml, __uint_as_float(erow[f.erow + i]));
+            ms = fmaxf(ms, __uint_as_float(erow[erow_total + f.erow + i]));
+        }
+        erow[f.erow + i] = __float_as_uint(ml);
+        erow[erow_total + f.erow + i] = __float_as_uint(ms);
     }
 }
 
@@ -922,82 +978,97 @@ __global__ void __launch_bounds__(kUpdThreads, 2) bk_update2_kernel(const FrontD
 
 // ---------------------------------------------------------------------------
 // inverses of the 64 x 64 diagonal blocks of the unit lower L11 (the sweeps'
-// dinv / dinvT blocks), one CTA of 64 threads per block
+// dinv / dinvT blocks), one CTA per block: the four 16 x 16 diagonal
+// sub-blocks by substitution (one column a thread), then the block rows
+// Linv_ij = -Linv_ii sum_{k=j}^{i-1} L_ik Linv_kj, thread (r, c) forming entry
+// (r, c) of every block of the row.  s_a holds L at c * ld + r and, once
+// formed, Linv(r, c) at the mirrored r * ld + c (r > c; unit diagonals).
 // ---------------------------------------------------------------------------
+constexpr int kDinvThreads = 256, kDinvLd = kTile + 1, kDinvSub = 16;
+
 template <class T, bool C>
-__global__ void __launch_bounds__(kTile) bk_dinv_kernel(const FrontDev* __restrict__ F, const int4* __restrict__ items,
-                                                        const T* __restrict__ L, T* __restrict__ dinv, T* __restrict__ dinvT) {
+__host__ __device__ constexpr size_t dinv_smem_bytes() {
+    return sizeof(V<T, C>) * (size_t)(kTile * kDinvLd + 3 * kDinvSub * kDinvSub);
+}
+
+template <class T, bool C>
+__global__ void __launch_bounds__(kDinvThreads) bk_dinv_kernel(const FrontDev* __restrict__ F, const int4* __restrict__ items,
+                                                               const T* __restrict__ L, T* __restrict__ dinv,
+                                                               T* __restrict__ dinvT) {
     using X = V<T, C>;
+    constexpr int ld = kDinvLd, sb = kDinvSub;
     extern __shared__ __align__(16) unsigned char bk_dinv_smem[];
-    X* s_a = reinterpret_cast<X*>(bk_dinv_smem);   // the block's strictly lower part, kTile x (kTile + 1)
+    X* s_a = reinterpret_cast<X*>(bk_dinv_smem);
+    X* s_g = s_a + kTile * ld;
     const int4 it = items[blockIdx.x];
     const FrontDev f = F[it.x];
     const int b = it.y, k = b * kTile, kb = min(kTile, f.n - k);
-    const int c = threadIdx.x;
-    for (int r = 0; r < kTile; ++r)
-        s_a[r + c * (kTile + 1)] = (r > c && r < kb && c < kb) ? ldv<T, C>(L, f.L + (k + r) + (int64_t)(k + c) * f.m) : X{};
+    const int tid = threadIdx.x;
+#pragma unroll 8
+    for (int idx = tid; idx < kTile * kTile; idx += kDinvThreads) {
+        const int r = idx % kTile, c = idx / kTile;
+        if (r > c) s_a[c * ld + r] = (r < kb && c < kb) ? ldv<T, C>(L, f.L + (k + r) + (int64_t)(k + c) * f.m) : X{};
+    }
     __syncthreads();
-    // column c of the inverse, written in place: x(c) = 1, x(r) = -sum_{c <= t < r} L(r, t) x(t)
-    X* Dv = reinterpret_cast<X*>(dinv) + f.dinv + (int64_t)b * kTile * kTile;
-    for (int r = 0; r < kTile; ++r) {
-        X x{};
-        if (c < kb && r == c) x = vone<X>();
-        else if (c < kb && r > c && r < kb) {
-            for (int t = c; t < r; ++t) mac(x, s_a[r + t * (kTile + 1)], Dv[t + c * kTile]);
-            x = neg(x);
+    if (tid < kTile) {   // column c of its sub-block's inverse: x(r) = -L(r, c) - sum_{c < t < r} L(r, t) x(t)
+        const int b0 = tid / sb * sb, c = tid % sb;
+        X x[sb];
+#pragma unroll
+        for (int r = 0; r < sb; ++r) {
+            X v = r > c ? s_a[(b0 + c) * ld + b0 + r] : X{};
+#pragma unroll
+            for (int t = 0; t < r; ++t)
+                if (t > c) mac(v, s_a[(b0 + t) * ld + b0 + r], x[t]);
+            x[r] = r > c ? neg(v) : X{};
         }
-        Dv[r + c * kTile] = x;
+#pragma unroll
+        for (int r = 0; r < sb; ++r)
+            if (r > c) s_a[(b0 + r) * ld + b0 + c] = x[r];
     }
-    if (dinvT) {
+    __syncthreads();
+    const int r = tid % sb, c = tid / sb;
+#pragma unroll
+    for (int i = 1; i < kTile / sb; ++i) {
+        if (sb * i >= kb) break;   // rows past the front's pivots
+        const int R = sb * i + r;
+        X acc[kTile / sb - 1];
+#pragma unroll
+        for (int j = 0; j < i; ++j) acc[j] = X{};
+#pragma unroll
+        for (int kk = 0; kk < i; ++kk) {
+#pragma unroll 4
+            for (int t = 0; t < sb; ++t) {
+                const X lik = s_a[(sb * kk + t) * ld + R];
+#pragma unroll
+                for (int j = 0; j <= kk; ++j) {
+                    const X lv = (j < kk || t > c) ? s_a[(sb * kk + t) * ld + sb * j + c] : t == c ? vone<X>() : X{};
+                    mac(acc[j], lik, lv);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < i; ++j) s_g[(j * sb + c) * sb + r] = acc[j];
         __syncthreads();
-        X* DvT = reinterpret_cast<X*>(dinvT) + f.dinv + (int64_t)b * kTile * kTile;
-        for (int idx = threadIdx.x; idx < kTile * kTile; idx += blockDim.x) {
-            const int cc = idx % kTile, i = idx / kTile;
-            DvT[cc + i * kTile] = Dv[i + cc * kTile];
+        for (int t = 0; t < r; ++t) {
+            const X lit = s_a[R * ld + sb * i + t];   // Linv_ii(r, t)
+#pragma unroll
+            for (int j = 0; j < i; ++j) mac(acc[j], lit, s_g[(j * sb + c) * sb + t]);
         }
+#pragma unroll
+        for (int j = 0; j < i; ++j) s_a[R * ld + sb * j + c] = neg(acc[j]);
+        __syncthreads();
     }
-}
-
-// ---------------------------------------------------------------------------
-// 2xFP16 split of a level's Schur complements on the tensor cores: largest
-// |component| of each row of L21 and of S21 = B = L21 D (D with its 2 x 2
-// blocks), over the front's n columns, into the two halves of erow (float
-// bits), one thread per row below the pivots
-// ---------------------------------------------------------------------------
-template <bool C, bool CJ>
-__global__ void __launch_bounds__(256) bk_rowmax_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl, int chunks,
-                                                        const float* __restrict__ L, const double* __restrict__ D,
-                                                        const double* __restrict__ E, uint32_t* __restrict__ erow, int64_t erow_total) {
-    using X = V<float, C>;
-    using W = DV<C>;
-    const int fi = blockIdx.x / chunks, ch = blockIdx.x % chunks;
-    const FrontDev f = F[fl[fi]];
-    const int i = f.n + ch * 256 + threadIdx.x;
-    if (i >= f.m) return;
-    const int64_t row = f.L + i;
-    float ml = 0.f, ms = 0.f;
-    X prev{}, cur = f.n > 0 ? ldv<float, C>(L, row) : X{};
-    X em1{};
-    for (int k = 0; k < f.n; ++k) {
-        const X next = k + 1 < f.n ? ldv<float, C>(L, row + (int64_t)(k + 1) * f.m) : X{};
-        const X d = conv<X>(reinterpret_cast<const W*>(D)[f.off + k]);
-        const X e = conv<X>(reinterpret_cast<const W*>(E)[f.off + k]);
-        X b = d * opc<CJ>(cur);
-        if (!is_zero(e)) b += opc<CJ>(e) * opc<CJ>(next);
-        if (!is_zero(em1)) b += em1 * opc<CJ>(prev);
-        if constexpr (C) {
-            ml = fmaxf(ml, fmaxf(fabsf(cur.r), fabsf(cur.i)));
-            ms = fmaxf(ms, fmaxf(fabsf(b.r), fabsf(b.i)));
-        } else {
-            ml = fmaxf(ml, fabsf(cur));
-            ms = fmaxf(ms, fabsf(b));
-        }
-        prev = cur;
-        cur = next;
-        em1 = e;
+    X* Dv = reinterpret_cast<X*>(dinv) + f.dinv + (int64_t)b * kTile * kTile;
+    X* DvT = dinvT ? reinterpret_cast<X*>(dinvT) + f.dinv + (int64_t)b * kTile * kTile : nullptr;
+    for (int idx = tid; idx < kTile * kTile; idx += kDinvThreads) {
+        const int lo = idx % kTile, hi = idx / kTile;
+        auto entry = [&](int i, int j) -> X {
+            if (i >= kb || j >= kb || i < j) return X{};
+            return i == j ? vone<X>() : s_a[i * ld + j];
+        };
+        Dv[idx] = entry(lo, hi);
+        if (DvT) DvT[idx] = entry(hi, lo);
     }
-    erow[f.erow + i] = __float_as_uint(ml);
-    erow[erow_total + f.erow + i] = __float_as_uint(ms);
 }
 
 // ---------------------------------------------------------------------------
@@ -1167,7 +1238,7 @@ static int level_t(Plan& P, int depth, cudaStream_t st, bool schur) {
         TRY((launch_panel<T, C, CJ>(P, fl, lv.nfronts, shape, L, cvec, vvec, st)));
         if (max_u > 0)
             bk_lower_kernel<T, C, CJ><<<(unsigned)((int64_t)lv.nfronts * chunks), kLowerRows, smem_lower, st>>>(
-                P.fronts, fl, chunks, L, P.D, P.E, P.pstate);
+                P.fronts, fl, chunks, L, P.D, P.E, P.pstate, std::is_same<T, float>::value ? P.erow : nullptr, P.erow_total);
         // every panel is at least kNb wide until the front is done, so the
         // trailing extents below bound the ones the kernels read from pstate
         int64_t tpf = 0;
@@ -1210,14 +1281,14 @@ static int level_t(Plan& P, int depth, cudaStream_t st, bool schur) {
 
 template <class T, bool C, bool CJ>
 static int finish_t(Plan& P, cudaStream_t st) {
-    const size_t smem = sizeof(V<T, C>) * kTile * (kTile + 1);
+    const size_t smem = dinv_smem_bytes<T, C>();
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(bk_dinv_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
     if (P.pivot_dinv_items > 0)
-        bk_dinv_kernel<T, C><<<(unsigned)P.pivot_dinv_items, kTile, smem, st>>>(P.fronts, reinterpret_cast<const int4*>(P.pivot_items),
+        bk_dinv_kernel<T, C><<<(unsigned)P.pivot_dinv_items, kDinvThreads, smem, st>>>(P.fronts, reinterpret_cast<const int4*>(P.pivot_items),
                                                                             reinterpret_cast<const T*>(P.L), reinterpret_cast<T*>(P.dinv),
                                                                             reinterpret_cast<T*>(P.dinvT));
     const unsigned g = grid1d(P.n, 256);
@@ -1288,24 +1359,6 @@ int pivot_level(Plan& P, int depth, cudaStream_t st, bool schur) {
     }
     if (!P.cplx()) return piv::level_t<float, false, false>(P, depth, st, schur);
     return cj ? piv::level_t<float, true, true>(P, depth, st, schur) : piv::level_t<float, true, false>(P, depth, st, schur);
-}
-
-// row maxima of the level's Schur operands for the 2xFP16 split (FP32 plans)
-int pivot_rowmax(Plan& P, int depth, cudaStream_t st) {
-    const SolveLevel& lv = P.solve_levels[depth];
-    if (lv.nfronts <= 0 || !P.erow || P.precision != CLIQ_FP32) return CLIQ_OK;
-    int max_u = 0;
-    for (int s : P.level_list[depth]) max_u = std::max(max_u, P.hfronts[s].m - P.hfronts[s].n);
-    if (max_u <= 0) return CLIQ_OK;
-    const int chunks = (max_u + 255) / 256;
-    const unsigned g = (unsigned)((int64_t)lv.nfronts * chunks);
-    const int32_t* fl = P.level_fronts + lv.fronts;
-    const float* L = reinterpret_cast<const float*>(P.L);
-    if (!P.cplx()) piv::bk_rowmax_kernel<false, false><<<g, 256, 0, st>>>(P.fronts, fl, chunks, L, P.D, P.E, P.erow, P.erow_total);
-    else if (P.conjugate) piv::bk_rowmax_kernel<true, true><<<g, 256, 0, st>>>(P.fronts, fl, chunks, L, P.D, P.E, P.erow, P.erow_total);
-    else piv::bk_rowmax_kernel<true, false><<<g, 256, 0, st>>>(P.fronts, fl, chunks, L, P.D, P.E, P.erow, P.erow_total);
-    P.total_launches += 1;
-    return check_cuda("pivoted row maxima");
 }
 
 int pivot_finish(Plan& P, cudaStream_t st) {
