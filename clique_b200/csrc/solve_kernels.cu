@@ -258,152 +258,249 @@ __global__ void __launch_bounds__(kSolveThreads) fwd_gather_kernel(const FrontDe
 }
 
 // ---------------------------------------------------------------------------
-// tiny fronts (one pivot block, at most kTinyLowerRows rows below): one warp
-// per front, kTinyWarps fronts per CTA, no flags.  Lane = pivot row / column
-// (lane and lane + 32); the right-hand-side rows a product needs are staged
-// in the warp's slice of shared memory and read as broadcasts.
-//   forward   x_T = L11^{-1} x_T,   W_B -= L21 x_T
-//   backward  z = x_T - op(L21)^T X[lowerStruct],   x_T = op(L11^{-1})^T z
+// tiny fronts (one pivot block, at most kTinyLowerRows rows below): one CTA
+// of four warps per front, no flags, the forward gather of the front included.
+//   forward   b = x_T + children,  x_T = L11^{-1} b,  W_B = children - L21 x_T
+//   backward  z = x_T - op(L21)^T X[lowerStruct],     x_T = op(L11^{-1})^T z
+// A front is 10 to 70 KB of loads and little arithmetic, so what bounds a
+// sweep of thousands of them is how many of a front's loads are in flight:
+// the four warps split every product's inner dimension, each issues eight
+// of its loads before it uses the first (the inverse's zero half is not
+// read), and the partial sums meet in shared memory.  L21 is read along its
+// rows in both sweeps; the backward one, which needs it by columns, stages it
+// through shared memory 32 rows at a time.  One warp per front, one column
+// after the other: 57 + 55 us for the leaves of 64 2D problems (8 complex FP32
+// columns), 68 + 40 us for those of a 30^3 grid (FP64); now 23 + 22 and 11 + 14.
 // ---------------------------------------------------------------------------
-constexpr int kTinyWarps = 8;
+constexpr int kTinyThreads = 128;
+constexpr int kTinyFly = 8;             // loads a thread issues before the first use
+constexpr int kTinyLd = 33;             // staged L21: 32 rows, one padding
+static_assert(kTinyThreads == 2 * kTile && kTinyLowerRows <= kTile, "two threads a pivot row");
 
+// shared memory: the right-hand sides [64][NR] and the partial sums
+// [4][NR][64], the backward sweep's staged L21 in the same place
 template <class T, bool C, int NR>
-__global__ void __launch_bounds__(32 * kTinyWarps) tiny_fwd_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
-                                                                   int nf, T* __restrict__ X, int64_t ldx, T* __restrict__ w0,
-                                                                   T* __restrict__ w1, const T* __restrict__ L,
-                                                                   const T* __restrict__ dinv, int nrhs) {
-    using Xv = V<T, C>;
-    extern __shared__ __align__(16) unsigned char tiny_smem[];
-    const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int fi = blockIdx.x * kTinyWarps + w;
-    if (fi >= nf) return;   // warp-uniform; only warp barriers below
-    Xv* sb = reinterpret_cast<Xv*>(tiny_smem) + (int64_t)w * kTile * NR;
-    const FrontDev f = F[fl[fi]];
-    const int n = f.n, u = f.m - f.n;
-    for (int e = lane; e < n * NR; e += 32) {
-        const int k = e % n, j = e / n;
-        sb[k * NR + j] = j < nrhs ? ldv<T, C>(X, f.off + k + (int64_t)j * ldx) : Xv{};
-    }
-    __syncwarp();
-    // x_T = L11^{-1} b: rows lane and lane + 32 (column k of the inverse is contiguous)
-    const Xv* Dv = reinterpret_cast<const Xv*>(dinv) + f.dinv;
+__host__ __device__ constexpr size_t tiny_smem_bytes() {
+    const size_t sums = (size_t)4 * NR * kTile, stage = (size_t)kTile * kTinyLd;
+    return sizeof(V<T, C>) * (kTile * NR + (sums > stage ? sums : stage));
+}
+
+// sum over k = w, w + 4, ... < n of M(row, k) s[k][:] for the rows lane and
+// lane + 32 of a 64-row column-major block, into the warp's partial sums.
+// LOW: M is lower triangular (rows < 32 end at column 31); else it is upper
+// triangular (rows >= 32 begin at column 32)
+template <bool LOW, bool CJ, int NR, class Xv>
+__device__ __forceinline__ void tiny_product(const Xv* M, int n, const Xv* s, Xv* red, int w, int lane) {
     Xv a0[NR], a1[NR];
 #pragma unroll
     for (int j = 0; j < NR; ++j) a0[j] = a1[j] = Xv{};
-    for (int k = 0; k < n; ++k) {
-        const Xv d0 = lane < n ? Dv[lane + k * kTile] : Xv{};
-        const Xv d1 = lane + 32 < n ? Dv[lane + 32 + k * kTile] : Xv{};
 #pragma unroll
-        for (int j = 0; j < NR; ++j) {
-            const Xv bv = sb[k * NR + j];
-            mac(a0[j], d0, bv);
-            mac(a1[j], d1, bv);
+    for (int half = 0; half < 2; ++half) {
+        const int kb = 32 * half;
+        if (kb >= n) break;
+        Xv d0[kTinyFly], d1[kTinyFly];
+#pragma unroll
+        for (int t = 0; t < kTinyFly; ++t) {
+            const int k = kb + w + 4 * t;
+            const bool r0 = LOW ? half == 0 : true, r1 = LOW ? true : half == 1;
+            d0[t] = (r0 && k < n && lane < n) ? M[lane + k * kTile] : Xv{};
+            d1[t] = (r1 && k < n && lane + 32 < n) ? M[lane + 32 + k * kTile] : Xv{};
+        }
+#pragma unroll
+        for (int t = 0; t < kTinyFly; ++t) {
+            const int k = kb + w + 4 * t;
+            if (k >= n) break;
+            const bool r0 = LOW ? half == 0 : true, r1 = LOW ? true : half == 1;
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                const Xv v = s[k * NR + j];
+                if (r0) mac(a0[j], opc<CJ>(d0[t]), v);
+                if (r1) mac(a1[j], opc<CJ>(d1[t]), v);
+            }
         }
     }
-    __syncwarp();
 #pragma unroll
     for (int j = 0; j < NR; ++j) {
-        if (lane < n) {
-            if (j < nrhs) stv<T, C>(X, f.off + lane + (int64_t)j * ldx, a0[j]);
-            sb[lane * NR + j] = a0[j];
+        red[(w * NR + j) * kTile + lane] = a0[j];
+        red[(w * NR + j) * kTile + lane + 32] = a1[j];
+    }
+}
+
+template <int NR, class Xv>
+__device__ __forceinline__ Xv tiny_sum(const Xv* red, int row, int j) {
+    return (red[j * kTile + row] + red[(NR + j) * kTile + row]) + (red[(2 * NR + j) * kTile + row] + red[(3 * NR + j) * kTile + row]);
+}
+
+template <class T, bool C, int NR>
+__global__ void __launch_bounds__(kTinyThreads) tiny_fwd_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
+                                                                T* __restrict__ X, int64_t ldx, T* __restrict__ w0,
+                                                                T* __restrict__ w1, const int32_t* __restrict__ cmaps,
+                                                                const T* __restrict__ L, const T* __restrict__ dinv, int nrhs) {
+    using Xv = V<T, C>;
+    extern __shared__ __align__(16) unsigned char tiny_smem[];
+    Xv* sb = reinterpret_cast<Xv*>(tiny_smem);
+    Xv* red = sb + kTile * NR;
+    const int tid = threadIdx.x, w = tid / 32, lane = tid % 32;
+    const FrontDev f = F[fl[blockIdx.x]];
+    const int n = f.n, u = f.m - f.n;
+    T* wb = f.pool == 0 ? w0 : w1;
+    const T* cw = f.pool == 0 ? w1 : w0;
+    const int32_t* lm = f.cmap >= 0 ? cmaps + f.cmap : nullptr;
+    // row i of the front: the children's contribution to right-hand side j
+    auto child = [&](int li, int ri, int j) -> Xv {
+        Xv v{};
+        if (li >= 0) v += ldv<T, C>(cw, f.CW[0] * nrhs + li + (int64_t)j * f.cu[0]);
+        if (ri >= 0) v += ldv<T, C>(cw, f.CW[1] * nrhs + ri + (int64_t)j * f.cu[1]);
+        return v;
+    };
+    {
+        const int i = tid % kTile;   // pivot row; half the right-hand sides a thread
+        const int li = (lm && i < n) ? lm[i] : -1, ri = (lm && i < n) ? lm[f.m + i] : -1;
+        Xv x[NR / 2];
+#pragma unroll
+        for (int q = 0; q < NR / 2; ++q) {
+            const int j = tid / kTile + 2 * q;
+            x[q] = (i < n && j < nrhs) ? ldv<T, C>(X, f.off + i + (int64_t)j * ldx) + child(li, ri, j) : Xv{};
         }
-        if (lane + 32 < n) {
-            if (j < nrhs) stv<T, C>(X, f.off + lane + 32 + (int64_t)j * ldx, a1[j]);
-            sb[(lane + 32) * NR + j] = a1[j];
+#pragma unroll
+        for (int q = 0; q < NR / 2; ++q) sb[i * NR + tid / kTile + 2 * q] = x[q];
+    }
+    // the children's contributions to the rows below (row r2, half the right-hand sides a thread)
+    const int r2 = tid % kTile;
+    Xv below[NR / 2];
+    {
+        const int li = (lm && r2 < u) ? lm[n + r2] : -1, ri = (lm && r2 < u) ? lm[f.m + n + r2] : -1;
+#pragma unroll
+        for (int q = 0; q < NR / 2; ++q) {
+            const int j = tid / kTile + 2 * q;
+            below[q] = (r2 < u && j < nrhs) ? child(li, ri, j) : Xv{};
         }
     }
-    __syncwarp();
-    // W_B -= L21 x_T, 32 rows at a time (row i of L21: stride m between columns)
-    T* wb = f.pool == 0 ? w0 : w1;
-    const Xv* Lf = reinterpret_cast<const Xv*>(L) + f.L + f.n;
-    for (int i0 = 0; i0 < u; i0 += 32) {
-        const int i = i0 + lane;
+    __syncthreads();
+    tiny_product<true, false, NR>(reinterpret_cast<const Xv*>(dinv) + f.dinv, n, sb, red, w, lane);
+    __syncthreads();
+    {
+        const int i = tid % kTile;
+#pragma unroll
+        for (int q = 0; q < NR / 2; ++q) {
+            const int j = tid / kTile + 2 * q;
+            const Xv v = tiny_sum<NR>(red, i, j);
+            sb[i * NR + j] = v;
+            if (i < n && j < nrhs) stv<T, C>(X, f.off + i + (int64_t)j * ldx, v);
+        }
+    }
+    if (u <= 0) return;
+    __syncthreads();
+    // L21 x_T: rows 32 (w & 1) + lane, columns k = w / 2, w / 2 + 2, ...
+    {
+        const Xv* Lf = reinterpret_cast<const Xv*>(L) + f.L + n;
+        const int i = 32 * (w & 1) + lane;
         Xv acc[NR];
 #pragma unroll
         for (int j = 0; j < NR; ++j) acc[j] = Xv{};
-        for (int k = 0; k < n; ++k) {
-            const Xv l = i < u ? Lf[i + (int64_t)k * f.m] : Xv{};
+        if (32 * (w & 1) < u) {
+            for (int k0 = w / 2; k0 < n; k0 += 2 * kTinyFly) {
+                Xv l[kTinyFly];
 #pragma unroll
-            for (int j = 0; j < NR; ++j) mac(acc[j], l, sb[k * NR + j]);
-        }
-        if (i < u) {
+                for (int t = 0; t < kTinyFly; ++t) l[t] = (i < u && k0 + 2 * t < n) ? Lf[i + (int64_t)(k0 + 2 * t) * f.m] : Xv{};
 #pragma unroll
-            for (int j = 0; j < NR; ++j) {
-                if (j >= nrhs) break;
-                const int64_t e = f.W * nrhs + i + (int64_t)j * f.u;
-                stv<T, C>(wb, e, ldv<T, C>(wb, e) - acc[j]);
+                for (int t = 0; t < kTinyFly; ++t) {
+                    if (k0 + 2 * t >= n) break;
+#pragma unroll
+                    for (int j = 0; j < NR; ++j) mac(acc[j], l[t], sb[(k0 + 2 * t) * NR + j]);
+                }
             }
+        }
+#pragma unroll
+        for (int j = 0; j < NR; ++j) red[((w / 2) * NR + j) * kTile + i] = acc[j];
+    }
+    __syncthreads();
+    if (r2 < u) {
+#pragma unroll
+        for (int q = 0; q < NR / 2; ++q) {
+            const int j = tid / kTile + 2 * q;
+            if (j < nrhs)
+                stv<T, C>(wb, f.W * nrhs + r2 + (int64_t)j * f.u, below[q] - (red[j * kTile + r2] + red[(NR + j) * kTile + r2]));
         }
     }
 }
 
 template <class T, bool C, bool CJ, int NR>
-__global__ void __launch_bounds__(32 * kTinyWarps) tiny_bwd_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
-                                                                   int nf, T* __restrict__ X, int64_t ldx, const T* __restrict__ L,
-                                                                   const T* __restrict__ dinvT, const int32_t* __restrict__ lower,
-                                                                   int nrhs) {
+__global__ void __launch_bounds__(kTinyThreads) tiny_bwd_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
+                                                                T* __restrict__ X, int64_t ldx, const T* __restrict__ L,
+                                                                const T* __restrict__ dinvT, const int32_t* __restrict__ lower,
+                                                                int nrhs) {
     using Xv = V<T, C>;
     extern __shared__ __align__(16) unsigned char tiny_smem[];
-    const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int fi = blockIdx.x * kTinyWarps + w;
-    if (fi >= nf) return;   // warp-uniform; only warp barriers below
-    Xv* sb = reinterpret_cast<Xv*>(tiny_smem) + (int64_t)w * kTile * NR;
-    const FrontDev f = F[fl[fi]];
+    Xv* sb = reinterpret_cast<Xv*>(tiny_smem);
+    Xv* red = sb + kTile * NR;
+    Xv* sl = red;                            // staged L21: column k at k * kTinyLd
+    const int tid = threadIdx.x, w = tid / 32, lane = tid % 32;
+    const FrontDev f = F[fl[blockIdx.x]];
     const int n = f.n, u = f.m - f.n;
-    Xv a0[NR], a1[NR];
+    const int i = tid % kTile, h = tid / kTile;   // pivot row / column, half of the work on it
+    Xv y[NR / 2];
 #pragma unroll
-    for (int j = 0; j < NR; ++j) {
-        a0[j] = (lane < n && j < nrhs) ? ldv<T, C>(X, f.off + lane + (int64_t)j * ldx) : Xv{};
-        a1[j] = (lane + 32 < n && j < nrhs) ? ldv<T, C>(X, f.off + lane + 32 + (int64_t)j * ldx) : Xv{};
+    for (int q = 0; q < NR / 2; ++q) {
+        const int j = h + 2 * q;
+        y[q] = (i < n && j < nrhs) ? ldv<T, C>(X, f.off + i + (int64_t)j * ldx) : Xv{};
     }
-    // z = y - op(L21)^T x_B, the solved rows below staged 32 at a time
-    const Xv* Lf = reinterpret_cast<const Xv*>(L) + f.L + f.n;
-    for (int i0 = 0; i0 < u; i0 += 32) {
-        const int i = i0 + lane;
+    // the solved rows below
+    {
         const int gi = i < u ? lower[f.lower + i] : -1;
-        __syncwarp();
+        Xv x[NR / 2];
 #pragma unroll
-        for (int j = 0; j < NR; ++j) sb[lane * NR + j] = (gi >= 0 && j < nrhs) ? ldv<T, C>(X, gi + (int64_t)j * ldx) : Xv{};
-        __syncwarp();
-        const int cn = min(32, u - i0);
-        for (int t = 0; t < cn; ++t) {
-            const Xv l0 = lane < n ? opc<CJ>(Lf[i0 + t + (int64_t)lane * f.m]) : Xv{};
-            const Xv l1 = lane + 32 < n ? opc<CJ>(Lf[i0 + t + (int64_t)(lane + 32) * f.m]) : Xv{};
+        for (int q = 0; q < NR / 2; ++q) {
+            const int j = h + 2 * q;
+            x[q] = (gi >= 0 && j < nrhs) ? ldv<T, C>(X, gi + (int64_t)j * ldx) : Xv{};
+        }
 #pragma unroll
-            for (int j = 0; j < NR; ++j) {
-                const Xv xv = sb[t * NR + j];
-                a0[j] -= l0 * xv;
-                a1[j] -= l1 * xv;
+        for (int q = 0; q < NR / 2; ++q) sb[i * NR + h + 2 * q] = x[q];
+    }
+    // op(L21)^T x_B: column i, rows t = h, h + 2, ... of each staged piece
+    Xv acc[NR];
+#pragma unroll
+    for (int j = 0; j < NR; ++j) acc[j] = Xv{};
+    const Xv* Lf = reinterpret_cast<const Xv*>(L) + f.L + n;
+    for (int t0 = 0; t0 < u; t0 += 32) {
+        const int cn = min(32, u - t0);
+        if (t0 > 0) __syncthreads();
+        for (int k0 = w; k0 < n; k0 += 4 * kTinyFly) {
+            Xv l[kTinyFly];
+#pragma unroll
+            for (int t = 0; t < kTinyFly; ++t)
+                l[t] = (lane < cn && k0 + 4 * t < n) ? Lf[t0 + lane + (int64_t)(k0 + 4 * t) * f.m] : Xv{};
+#pragma unroll
+            for (int t = 0; t < kTinyFly; ++t)
+                if (k0 + 4 * t < n) sl[(k0 + 4 * t) * kTinyLd + lane] = l[t];
+        }
+        __syncthreads();
+        if (i < n) {
+            for (int t = h; t < cn; t += 2) {
+                const Xv l = opc<CJ>(sl[i * kTinyLd + t]);
+#pragma unroll
+                for (int j = 0; j < NR; ++j) mac(acc[j], l, sb[(t0 + t) * NR + j]);
             }
         }
     }
-    __syncwarp();
+    __syncthreads();
+    // z into sb (the halves' sums meet in red)
 #pragma unroll
-    for (int j = 0; j < NR; ++j) {
-        if (lane < n) sb[lane * NR + j] = a0[j];
-        if (lane + 32 < n) sb[(lane + 32) * NR + j] = a1[j];
+    for (int j = 0; j < NR; ++j) red[(h * NR + j) * kTile + i] = acc[j];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NR / 2; ++q) {
+        const int j = h + 2 * q;
+        sb[i * NR + j] = y[q] - (red[j * kTile + i] + red[(NR + j) * kTile + i]);
     }
-    __syncwarp();
+    __syncthreads();
     // x_T[k] = sum_t op(Linv[t][k]) z[t]; Linv[t][k] is element k + 64 t of the row-major copy
-    const Xv* DvT = reinterpret_cast<const Xv*>(dinvT) + f.dinv;
-    Xv r0[NR], r1[NR];
+    tiny_product<false, CJ, NR>(reinterpret_cast<const Xv*>(dinvT) + f.dinv, n, sb, red, w, lane);
+    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < NR; ++j) r0[j] = r1[j] = Xv{};
-    for (int t = 0; t < n; ++t) {
-        const Xv d0 = lane < n ? opc<CJ>(DvT[lane + t * kTile]) : Xv{};
-        const Xv d1 = lane + 32 < n ? opc<CJ>(DvT[lane + 32 + t * kTile]) : Xv{};
-#pragma unroll
-        for (int j = 0; j < NR; ++j) {
-            const Xv zv = sb[t * NR + j];
-            mac(r0[j], d0, zv);
-            mac(r1[j], d1, zv);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-        if (j >= nrhs) break;
-        if (lane < n) stv<T, C>(X, f.off + lane + (int64_t)j * ldx, r0[j]);
-        if (lane + 32 < n) stv<T, C>(X, f.off + lane + 32 + (int64_t)j * ldx, r1[j]);
+    for (int q = 0; q < NR / 2; ++q) {
+        const int j = h + 2 * q;
+        if (i < n && j < nrhs) stv<T, C>(X, f.off + i + (int64_t)j * ldx, tiny_sum<NR>(red, i, j));
     }
 }
 
@@ -1244,7 +1341,7 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
     using Xv = V<T, C>;
     const size_t smem_fwd = sizeof(Xv) * (4 + kQ) * kTile * NR;
     const size_t smem_bwd = sizeof(Xv) * ((3 + kQ) * kTile * NR + kTile * (kTile + 1)) + sizeof(int32_t) * kLowerChunkTiles * kTile;
-    const size_t smem_tiny = sizeof(Xv) * kTinyWarps * kTile * NR;
+    constexpr size_t smem_tiny = tiny_smem_bytes<T, C, NR>();
     static bool attr_done = false;
     if (!attr_done) {
         cudaFuncSetAttribute(fwd_sweep_kernel<T, C, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fwd);
@@ -1282,12 +1379,15 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
     for (int d = P.max_depth; d >= 0; --d) {
         const SolveLevel& lv = P.solve_levels[d];
         if (lv.nfronts == 0) continue;
-        fwd_gather_kernel<T, C><<<dim3(lv.nfronts, lv.gather_chunks), kSolveThreads, 0, P.stream>>>(
-            P.fronts, P.level_fronts + lv.fronts, X, P.n, w0, w1, P.cmaps, nrhs);
-        ++launches;
+        const int nbig = lv.nfronts - lv.ntiny;   // the level's tiny fronts are the last of its list
+        if (nbig > 0) {
+            fwd_gather_kernel<T, C><<<dim3(nbig, lv.gather_chunks), kSolveThreads, 0, P.stream>>>(
+                P.fronts, P.level_fronts + lv.fronts, X, P.n, w0, w1, P.cmaps, nrhs);
+            ++launches;
+        }
         if (lv.ntiny > 0) {
-            tiny_fwd_kernel<T, C, NR><<<(lv.ntiny + kTinyWarps - 1) / kTinyWarps, 32 * kTinyWarps, smem_tiny, P.stream>>>(
-                P.fronts, P.tiny_fronts + lv.tiny, lv.ntiny, X, P.n, w0, w1, reinterpret_cast<const T*>(P.L),
+            tiny_fwd_kernel<T, C, NR><<<lv.ntiny, kTinyThreads, smem_tiny, P.stream>>>(
+                P.fronts, P.level_fronts + lv.fronts + nbig, X, P.n, w0, w1, P.cmaps, reinterpret_cast<const T*>(P.L),
                 reinterpret_cast<const T*>(P.dinv), nrhs);
             ++launches;
         }
@@ -1305,8 +1405,8 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
     for (int d = 0; d <= P.max_depth; ++d) {
         const SolveLevel& lv = P.solve_levels[d];
         if (lv.ntiny > 0) {
-            tiny_bwd_kernel<T, C, CJ, NR><<<(lv.ntiny + kTinyWarps - 1) / kTinyWarps, 32 * kTinyWarps, smem_tiny, P.stream>>>(
-                P.fronts, P.tiny_fronts + lv.tiny, lv.ntiny, X, P.n, reinterpret_cast<const T*>(P.L),
+            tiny_bwd_kernel<T, C, CJ, NR><<<lv.ntiny, kTinyThreads, smem_tiny, P.stream>>>(
+                P.fronts, P.level_fronts + lv.fronts + lv.nfronts - lv.ntiny, X, P.n, reinterpret_cast<const T*>(P.L),
                 reinterpret_cast<const T*>(P.dinvT), P.lower, nrhs);
             ++launches;
         }

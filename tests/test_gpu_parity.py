@@ -685,7 +685,7 @@ def test_refined_solve_fp64_fallback():
 @pytest.mark.parametrize("nrhs", [3, 9, 20])
 def test_tiny_front_sweeps_match_oracle(oracle, kind, nrhs):
     """A 2D grid whose leaves have one pivot block and at most 64 rows below
-    (the one-warp-per-front sweeps) solved in FP64 for 3, 9 and 20
+    (the tiny-front sweeps) solved in FP64 for 3, 9 and 20
     right-hand sides (the 4-, 16- and 16 + 4-column sweep instantiations),
     against the oracle's solve on the same ordering."""
     n1, n2, cutoff = 41, 37, 32
@@ -712,3 +712,21 @@ def test_tiny_front_sweeps_match_oracle(oracle, kind, nrhs):
     assert F.ldl(96) == 0
     assert rel(X, F.solve(B.copy(order="F"))) <= 1e-10
     assert residual(A, X, B) <= 1e-11
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("nrhs", [1, 5, 16])
+@pytest.mark.parametrize("dims,cutoff", [((1, 1, 1), 1), ((31, 3, 1), 31), ((97, 2, 1), 32), ((66, 5, 1), 33), ((27, 14, 1), 63),
+                                         ((26, 20, 1), 64), ((9, 9, 9), 65)])
+def test_tiny_front_sizes(oracle, kind, nrhs, dims, cutoff):
+    """Fronts of 1 .. 64 pivots with 0 .. 64 rows below, beside larger ones at
+    the same depth (65 pivots and more take the general sweeps): the oracle's
+    solution to 1e-10, as the other solves."""
+    A = ops.laplacian_3d(*dims, 6.1) if kind == "real" else ops.helmholtz_pml_3d(*dims, omega=9.0, b=2)
+    _, info, L = build(A, dims, cutoff)
+    B = ops.random_rhs(A.n, nrhs, seed=nrhs, complex_=kind == "complex")
+    X = cliq.Solve(info, L, B.copy(order="F"))
+    S = oracle.Symbolic(*dims, A.rowptr, A.colind, cutoff=cutoff)
+    F = oracle.Fronts(S, A.values, is_complex=kind == "complex")
+    assert F.ldl(96) == 0
+    assert rel(X, F.solve(B.copy(order="F"))) <= 1e-10
