@@ -48,8 +48,11 @@ void set_last_error(const std::string& msg);
 constexpr int kTile = 64;        // rows per solve block, GEMM tile edge
 constexpr int kTcBM = 128;       // tensor-core update tile: rows
 constexpr int kTcBN = 128;       // tensor-core update tile: columns (two CTAs per SM at 128)
-constexpr int kEACols = 16;      // columns per extend-add work item
-constexpr int kEARows = 2048;    // rows per extend-add work item
+constexpr int kEACols = 16;      // most columns per extend-add work item
+constexpr int kEAMinCols = 2;    // fewest, on levels of few items
+constexpr int kEAItems = 1184;   // items that fill the device: 148 SMs x 8 resident CTAs
+constexpr int kEARows = 2048;    // rows per extend-add work item (over kEAGroups where that many columns are swept at a time)
+constexpr int kEAGroups = 4;     // columns swept at a time on levels of short fronts
 // Triangular sweeps: the worker of pivot block s adds the contributions of
 // the solved blocks up to s - kSolveLag and applies the block's inverse; the
 // chain CTA of the front adds the newest block (s - 1) through the stored
@@ -121,7 +124,7 @@ struct Launch {
     int32_t nitems;
     int64_t prefix;       // GEMM: offset into the tile prefix array
     int64_t nblocks;      // grid size
-    int32_t k;            // DIAG / PANEL: column offset of the step
+    int32_t k;            // DIAG / PANEL: column offset of the step; EXTEND_ADD: columns swept at a time
     int32_t depth;
     double work;          // GEMM: algorithmic flops; EXTEND_ADD: algorithmic bytes
     int32_t schur;        // GEMM: 1 for the Schur-complement update, 0 for an in-panel update

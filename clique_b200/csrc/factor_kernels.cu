@@ -47,22 +47,32 @@ __device__ __forceinline__ float cabsmax(cx<double> v) { return (float)fmax(fabs
 // ---------------------------------------------------------------------------
 // 1. extend-add (gather form)
 //
-// Work item (front, j0, i0): columns j0 .. j0+15, rows i0 .. i0+kEARows-1 on
-// or below the diagonal.  The children's maps of the item's rows and
-// columns are staged in shared memory once; the CTA then sweeps one column at a time
-// down a contiguous run of rows (consecutive threads, consecutive rows: few
-// DRAM pages open per CTA), each thread issuing the gathers of all its rows
-// of the column before any store.
+// Work item (front, j0, i0, columns): the item's columns from j0 on, its rows
+// from i0 on (kEARows of them, or a quarter) on or below the diagonal.  The
+// children's maps of the item's rows and columns are staged in shared memory
+// once; the CTA (or each of four thread groups, where the level's fronts are
+// short) then sweeps one column at a time down a contiguous run of rows
+// (consecutive threads, consecutive rows: few DRAM pages open per CTA), each
+// thread issuing the gathers of all its rows of the column before any store.
+// What bounds an item is that chain of columns, one gather latency each, so
+// the schedule takes items of fewer columns on levels whose CTAs would not
+// fill the device otherwise (plan.cu).  All levels, one column at a time and
+// 16 columns an item: 30^3 FP64 373 us, 701 x 503 FP64 987 us, 12 x 11 x 9 95 us;
+// so: 182, 500 and 32 us.
 // ---------------------------------------------------------------------------
 constexpr int kEAPer = kEARows / kThreads;   // rows of a column per thread
 static_assert(kEARows % kThreads == 0, "whole rows per thread");
 
-template <class T, bool C>
+// LANES threads to a column: kThreads, or a quarter of them on levels of short
+// fronts.  Two kernels, because with the stride as a variable, or both strides
+// in one kernel, the large levels take 16 to 35 % longer.
+template <class T, bool C, int LANES>
 __global__ void __launch_bounds__(kThreads) extend_add_kernel(const FrontDev* __restrict__ F, const int4* __restrict__ items,
                                                               T* __restrict__ L, T* __restrict__ pool0, T* __restrict__ pool1,
                                                               const int32_t* __restrict__ cmaps) {
     using X = V<T, C>;
-    __shared__ int32_t s_map[2][kEARows];
+    constexpr int kRows = kEAPer * LANES;
+    __shared__ int32_t s_map[2][kRows];
     __shared__ int32_t s_cmap[2][kEACols];
     const int4 it = items[blockIdx.x];
     const FrontDev f = F[it.x];
@@ -71,8 +81,8 @@ __global__ void __launch_bounds__(kThreads) extend_add_kernel(const FrontDev* __
     const T* cp = f.pool == 0 ? pool1 : pool0;
     const int32_t* lm = f.cmap >= 0 ? cmaps + f.cmap : nullptr;
     const int32_t* rm = lm ? lm + f.m : nullptr;
-    const int i_end = min(f.m, i0 + kEARows);
-    const int j_end = min(f.m, j0 + kEACols);
+    const int i_end = min(f.m, i0 + kRows);
+    const int j_end = min(f.m, j0 + it.w);
     for (int i = max(j0, i0) + threadIdx.x; i < i_end; i += kThreads) {
         s_map[0][i - i0] = lm ? lm[i] : -1;
         s_map[1][i - i0] = rm ? rm[i] : -1;
@@ -83,13 +93,13 @@ __global__ void __launch_bounds__(kThreads) extend_add_kernel(const FrontDev* __
         s_cmap[1][threadIdx.x] = (rm && j < j_end) ? rm[j] : -1;
     }
     __syncthreads();
-    for (int j = j0; j < j_end; ++j) {
+    for (int j = LANES == kThreads ? j0 : j0 + (int)threadIdx.x / LANES; j < j_end; j += kThreads / LANES) {
         const int lj = s_cmap[0][j - j0], rj = s_cmap[1][j - j0];
-        const int ib = max(j, i0) + threadIdx.x;
+        const int ib = max(j, i0) + threadIdx.x % LANES;
         X v[kEAPer];
 #pragma unroll
         for (int u = 0; u < kEAPer; ++u) {
-            const int i = ib + u * kThreads;
+            const int i = ib + u * LANES;
             X t = X{};
             if (i < i_end) {
                 const int li = lj >= 0 ? s_map[0][i - i0] : -1, ri = rj >= 0 ? s_map[1][i - i0] : -1;
@@ -100,12 +110,21 @@ __global__ void __launch_bounds__(kThreads) extend_add_kernel(const FrontDev* __
         }
 #pragma unroll
         for (int u = 0; u < kEAPer; ++u) {
-            const int i = ib + u * kThreads;
+            const int i = ib + u * LANES;
             if (i >= i_end) break;
             if (j < f.n) stv<T, C>(L, f.L + i + (int64_t)j * f.m, v[u]);
             else stv<T, C>(up, f.U + (i - f.n) + (int64_t)(j - f.n) * f.u, v[u]);
         }
     }
+}
+
+template <class T, bool C>
+static void launch_extend_add(const Plan& P, const Launch& ln, T* L, T* p0, T* p1, const int32_t* cmaps, cudaStream_t st) {
+    const int4* items = reinterpret_cast<const int4*>(P.items) + ln.items;
+    if (ln.k == 1)   // one column at a time
+        extend_add_kernel<T, C, kThreads><<<(unsigned)ln.nblocks, kThreads, 0, st>>>(P.fronts, items, L, p0, p1, cmaps);
+    else
+        extend_add_kernel<T, C, kThreads / kEAGroups><<<(unsigned)ln.nblocks, kThreads, 0, st>>>(P.fronts, items, L, p0, p1, cmaps);
 }
 
 // ---------------------------------------------------------------------------
@@ -356,12 +375,23 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(const FrontDev* __restr
     const int r0 = k + kb + kTile * rb;
     const int rows = min(kTile, f.m - r0);
     const X* U = reinterpret_cast<const X*>(tinv) + (int64_t)slot * nb * nb;
-    for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) sU[idx] = U[idx];
-    for (int idx = threadIdx.x; idx < kTile * nb; idx += blockDim.x) {
-        const int r = idx % kTile, t = idx / kTile;
-        X v{};
-        if (r < rows && t < kb) v = ldv<T, C>(L, f.L + (r0 + r) + (int64_t)(k + t) * f.m);
-        sA[r * ldA + t] = v;
+    // all loads of a thread before the first one is used: the tile's, then U's
+    constexpr int kPer = nb * nb / kThreads;
+    static_assert(kTile == nb && kPer * kThreads == nb * nb, "whole entries per thread");
+    {
+        X v[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const int r = threadIdx.x % kTile, t = threadIdx.x / kTile + (kThreads / kTile) * q;
+            v[q] = (r < rows && t < kb) ? ldv<T, C>(L, f.L + (r0 + r) + (int64_t)(k + t) * f.m) : X{};
+        }
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+            sA[(threadIdx.x % kTile) * ldA + threadIdx.x / kTile + (kThreads / kTile) * q] = v[q];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) v[q] = U[threadIdx.x + kThreads * q];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) sU[threadIdx.x + kThreads * q] = v[q];
     }
     if (threadIdx.x < kb) {
         const W d = reinterpret_cast<const W*>(D)[f.off + k + threadIdx.x];
@@ -697,7 +727,7 @@ static int64_t issue_factor(Plan& P, bool captured = false) {
         if (P.profile) cudaEventRecord(P.events[3 * li], st);
         switch (ln.kind) {
             case Launch::EXTEND_ADD:
-                extend_add_kernel<T, C><<<(unsigned)ln.nblocks, kThreads, 0, st>>>(P.fronts, items + ln.items, L, p0, p1, P.cmaps);
+                launch_extend_add<T, C>(P, ln, L, p0, p1, P.cmaps, st);
                 launch_assemble_level(P, ln.depth, st);   // A's entries of this level's fronts
                 break;
             case Launch::DIAG:
@@ -801,7 +831,7 @@ static int issue_factor_pivoted(Plan& P, int64_t* nlaunch) {
     }
     for (const Launch& ln : P.launches) {
         if (ln.kind != Launch::EXTEND_ADD || ln.nblocks <= 0) continue;
-        extend_add_kernel<T, C><<<(unsigned)ln.nblocks, kThreads, 0, st>>>(P.fronts, items + ln.items, L, p0, p1, P.cmaps_orig);
+        launch_extend_add<T, C>(P, ln, L, p0, p1, P.cmaps_orig, st);
         ++launches;
         TRY(launch_assemble_level(P, ln.depth, st));
         const bool on_tc = tc_ok[ln.depth] != 0;

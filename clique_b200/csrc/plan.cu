@@ -360,13 +360,31 @@ int build_plan(Plan& P, const cliq_symm_info* info, int64_t n, const int32_t* ma
             Launch ln{};
             ln.kind = Launch::EXTEND_ADD;
             ln.items = (int64_t)items.size() / 4;
+            // every front, leaves included: the extend-add writes each lower
+            // entry (the fronts are not cleared beforehand).  An item's time is
+            // its columns' gather latencies one after the other: levels of
+            // short fronts (a column of theirs gives most threads no row)
+            // sweep kEAGroups columns at a time, and a level of fewer than
+            // kEAItems items takes fewer columns an item
+            int maxm = 0;
+            for (int s : lv) maxm = std::max(maxm, P.hfronts[s].m);
+            const int groups = maxm <= kEARows / kEAGroups ? kEAGroups : 1, rows = kEARows / groups;
+            auto items_of = [&](int cols) {
+                int64_t t = 0;
+                for (int s : lv) {
+                    const int m = P.hfronts[s].m;
+                    for (int j0 = 0; j0 < m; j0 += cols) t += (m - j0 / rows * rows + rows - 1) / rows;
+                }
+                return t;
+            };
+            int cols = kEACols;
+            while (cols > std::max(kEAMinCols, groups) && items_of(cols) < kEAItems) cols /= 2;
             for (int s : lv) {
-                const FrontDev& f = P.hfronts[s];
-                // every front, leaves included: the extend-add writes each lower
-                // entry (the fronts are not cleared beforehand)
-                for (int j0 = 0; j0 < f.m; j0 += kEACols)
-                    for (int i0 = j0 / kEARows * kEARows; i0 < f.m; i0 += kEARows) push_item(s, j0, i0, 0);
+                const int m = P.hfronts[s].m;
+                for (int j0 = 0; j0 < m; j0 += cols)
+                    for (int i0 = j0 / rows * rows; i0 < m; i0 += rows) push_item(s, j0, i0, cols);
             }
+            ln.k = groups;
             ln.nitems = (int32_t)(items.size() / 4 - ln.items);
             ln.nblocks = ln.nitems;
             ln.depth = d;
