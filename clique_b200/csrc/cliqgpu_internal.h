@@ -59,6 +59,7 @@ constexpr int kEAGroups = 4;     // columns swept at a time on levels of short f
 // product of that inverse with the coupling tile.
 constexpr int kSolveLag = 2;
 constexpr int kSolveRhsChunk = 16;   // right-hand sides per sweep (partial-sum stride)
+constexpr int kGatherRows = 256;     // front rows per gather CTA (grid y of the gather launch)
 constexpr int kLowerChunkTiles = 16; // backward: 64-row tiles below the pivots per helper
 // sweep work items {front, kind, block, chunk}
 enum SweepItem : int { kItemChain = 0, kItemPivotRows = 1, kItemLowerRows = 2, kItemColumns = 1, kItemLowerChunk = 2,
@@ -173,7 +174,7 @@ struct SolveLevel {
     int64_t bwd_items;
     int32_t nbwd;
     int32_t depth;
-    int32_t gather_chunks;   // 1024-row chunks of the level's tallest front (gather grid y)
+    int32_t gather_chunks;   // kGatherRows-row chunks of the level's tallest front (gather grid y)
     int32_t ntiny;           // the last of the level's fronts: tiny ones, swept by kernels of their own
 };
 

@@ -581,7 +581,7 @@ int build_plan(Plan& P, const cliq_symm_info* info, int64_t n, const int32_t* ma
         sl.fronts = (int64_t)level_fronts.size();
         sl.nfronts = (int32_t)P.level_list[d].size();
         sl.gather_chunks = 1;
-        for (int s : P.level_list[d]) sl.gather_chunks = std::max(sl.gather_chunks, (P.hfronts[s].m + 1023) / 1024);
+        for (int s : P.level_list[d]) sl.gather_chunks = std::max(sl.gather_chunks, (P.hfronts[s].m + kGatherRows - 1) / kGatherRows);
         // forward: each front's chain followed by its pivot-row workers in the
         // order the chain consumes their results, then the workers for the
         // rows below the pivots (they only wait on chains, all issued before)

@@ -50,7 +50,6 @@ constexpr int kE = kTile / kQ;              // tile elements per thread and slic
 constexpr int kLag = kSolveLag;             // worker s adds the blocks t <= s - kLag
 constexpr int kMaxRhsChunk = kSolveRhsChunk;   // right-hand sides per sweep
 constexpr int kPartialStride = kTile * kMaxRhsChunk;   // elements per pivot block in the partial store
-constexpr int kGatherRows = 1024;           // front rows per gather CTA (grid y of the gather launch)
 constexpr uint64_t kSpinNs = 500000000ull;  // 0.5 s bound on any single wait
 
 __device__ __forceinline__ int ld_acquire(const int32_t* p) {
@@ -223,36 +222,47 @@ __device__ __forceinline__ void put_x(const Xv (&xr)[XStage<NR>::kN], Xv* s) {
 }
 
 // ---------------------------------------------------------------------------
-// forward gather: X_T += children's W_B (rows < n), W_B := children's W_B
+// forward gather: X_T += children's W_B (rows < n), W_B := children's W_B.
+// One row a thread: its children's rows are looked up once, and the loads of
+// kGatherFly right-hand sides are issued before the first is used (what bounds
+// a launch on the levels of few fronts is that chain of loads: 79 us for 9090
+// rows and 16 columns when a thread took rows and columns one by one, 14 us so)
 // ---------------------------------------------------------------------------
+constexpr int kGatherFly = 4;
+static_assert(kGatherRows == kSolveThreads, "one row per thread");
+
 template <class T, bool C>
 __global__ void __launch_bounds__(kSolveThreads) fwd_gather_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
                                                                    T* __restrict__ X, int64_t ldx, T* __restrict__ w0, T* __restrict__ w1,
                                                                    const int32_t* __restrict__ cmaps, int nrhs) {
     using Xv = V<T, C>;
     const FrontDev f = F[fl[blockIdx.x]];
-    const int i0 = blockIdx.y * kGatherRows;       // this CTA's chunk of the front's rows
-    if (i0 >= f.m) return;
-    const int ni = min(kGatherRows, f.m - i0);
+    const int i = blockIdx.y * kGatherRows + threadIdx.x;
+    if (i >= f.m) return;
+    const bool top = i < f.n;
+    if (top && f.cmap < 0) return;
     T* wb = f.pool == 0 ? w0 : w1;
     const T* cw = f.pool == 0 ? w1 : w0;
-    const int32_t* lm = f.cmap >= 0 ? cmaps + f.cmap : nullptr;
-    const int32_t* rm = lm ? lm + f.m : nullptr;
-    const int64_t total = (int64_t)ni * nrhs;
-    for (int64_t idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int i = i0 + (int)(idx % ni), j = (int)(idx / ni);
-        if (i < f.n && !lm) continue;
-        Xv v{};
-        if (lm) {
-            const int li = lm[i], ri = rm[i];
-            if (li >= 0) v += ldv<T, C>(cw, f.CW[0] * nrhs + li + (int64_t)j * f.cu[0]);
-            if (ri >= 0) v += ldv<T, C>(cw, f.CW[1] * nrhs + ri + (int64_t)j * f.cu[1]);
+    const int li = f.cmap >= 0 ? cmaps[f.cmap + i] : -1, ri = f.cmap >= 0 ? cmaps[f.cmap + f.m + i] : -1;
+    const int64_t l0 = f.CW[0] * nrhs + li, r0 = f.CW[1] * nrhs + ri;
+    const int64_t x0 = f.off + i, b0 = f.W * nrhs + (i - f.n);
+    for (int j0 = 0; j0 < nrhs; j0 += kGatherFly) {
+        Xv x[kGatherFly], l[kGatherFly], r[kGatherFly];
+#pragma unroll
+        for (int t = 0; t < kGatherFly; ++t) {
+            const int j = j0 + t;
+            const bool in = j < nrhs;
+            x[t] = (in && top) ? ldv<T, C>(X, x0 + (int64_t)j * ldx) : Xv{};
+            l[t] = (in && li >= 0) ? ldv<T, C>(cw, l0 + (int64_t)j * f.cu[0]) : Xv{};
+            r[t] = (in && ri >= 0) ? ldv<T, C>(cw, r0 + (int64_t)j * f.cu[1]) : Xv{};
         }
-        if (i < f.n) {
-            const int64_t e = f.off + i + (int64_t)j * ldx;
-            stv<T, C>(X, e, ldv<T, C>(X, e) + v);
-        } else {
-            stv<T, C>(wb, f.W * nrhs + (i - f.n) + (int64_t)j * f.u, v);
+#pragma unroll
+        for (int t = 0; t < kGatherFly; ++t) {
+            const int j = j0 + t;
+            if (j >= nrhs) break;
+            const Xv v = l[t] + r[t];
+            if (top) stv<T, C>(X, x0 + (int64_t)j * ldx, x[t] + v);
+            else stv<T, C>(wb, b0 + (int64_t)j * f.u, v);
         }
     }
 }
