@@ -71,18 +71,19 @@ template <class T> __device__ __forceinline__ void mac(cx<T>& acc, cx<T> a, cx<T
 }
 
 // Reciprocal of a pivot, on the critical path of every elimination step.
-// 1/x for x within float range: Newton-Raphson iteration y <- y (2 - x y)
-// from the single-precision reciprocal (about 23 correct bits, two steps
-// give full double precision); outside that range the IEEE reciprocal.
+// 1/x for x within float range: one third-order step y + y (e + e^2),
+// e = 1 - x y, from the hardware's approximate reciprocal (relative error
+// below 2^-19, so e^3 is below the last bit; three dependent operations where
+// two Newton steps take four); outside that range the IEEE reciprocal.
 // Complex: conj(d) / |d|^2, with d scaled by a power of two when |d|^2
 // would leave the range.
 __device__ __forceinline__ double recip_nr(double x) {
     const double ax = fabs(x);
     if (!(ax > 1e-30 && ax < 1e30)) return __drcp_rn(x);
-    double y = (double)__frcp_rn((float)x);
-    y = y * fma(-x, y, 2.0);
-    y = y * fma(-x, y, 2.0);
-    return y;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ float pivot_recip(float d) { return __frcp_rn(d); }
 __device__ __forceinline__ cx<float> pivot_recip(cx<float> d) {
@@ -111,6 +112,14 @@ __device__ __forceinline__ cx<double> pivot_recip(cx<double> d) {
     const double xr = d.r * sc, xi = d.i * sc;
     const double s = __drcp_rn(fma(xr, xr, xi * xi)) * sc;
     return {xr * s, -xi * s};
+}
+
+// acc -= a*b
+__device__ __forceinline__ void nmac(float& acc, float a, float b) { acc = fmaf(-a, b, acc); }
+__device__ __forceinline__ void nmac(double& acc, double a, double b) { acc = fma(-a, b, acc); }
+template <class T> __device__ __forceinline__ void nmac(cx<T>& acc, cx<T> a, cx<T> b) {
+    acc.r = fma(-a.r, b.r, acc.r); acc.r = fma(a.i, b.i, acc.r);
+    acc.i = fma(-a.r, b.i, acc.i); acc.i = fma(-a.i, b.r, acc.i);
 }
 
 // element load / store from a T* arena

@@ -137,7 +137,9 @@ static void launch_extend_add(const Plan& P, const Launch& ln, T* L, T* p0, T* p
 // one barrier per pivot, the working copies double-buffered by pivot
 // parity, and the reciprocal of the next pivot computed by its owner right
 // after its own update, so the per-pivot critical path is one update, one
-// reciprocal and one barrier.  Then G = A_ip op(L_pp^{-1})^T,
+// reciprocal and one barrier (a warp's instruction stream, about six cycles an
+// instruction with two warps a scheduler, is what the kernel takes; holding the
+// block in registers, four pivots a barrier, took 39 us where this takes 25).  Then G = A_ip op(L_pp^{-1})^T,
 // L_ip = G D_p^{-1} and the rank-16 update A_22 -= G op(L_2p)^T (2 x 2
 // register tiles).  Finally the off-diagonal 16 x 16 blocks of L^{-1}:
 //   Linv_ij = -Linv_ii * sum_{k=j}^{i-1} L_ik Linv_kj,   i > j.
@@ -230,9 +232,9 @@ __global__ void __launch_bounds__(kThreads, 2) diag_ldl_kernel(const FrontDev* _
                 const W rd = s_rd[b0 + j];
                 const W prj = P0[j * kSubLd + sr];                  // P[r][j]
                 const W lrj = prj * rd;
-                if (sc > j) a -= lrj * P0[sc * kSubLd + j];          // P[r][c] -= L[r][j] P[j][c]
+                if (sc > j) nmac(a, lrj, P0[sc * kSubLd + j]);          // P[r][c] -= L[r][j] P[j][c]
                 else if (sc == j) a = lrj;
-                x -= lrj * X0[sc * kSubLd + j];                      // row r -= L[r][j] row j
+                nmac(x, lrj, X0[sc * kSubLd + j]);                      // row r -= L[r][j] row j
             }
             P1[sc * kSubLd + sr] = a;
             X1[sc * kSubLd + sr] = x;
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(kThreads, 2) diag_ldl_kernel(const FrontDev* _
         for (int idx = tid; idx < R * kSub; idx += kThreads) {
             const int i = i0 + idx % R, c = idx / R;
             W g = sA[(b0 + c) * ld + i];
-            for (int t = 0; t < c; ++t) g += sA[(b0 + t) * ld + i] * opc<CJ>(sA[(b0 + c) * ld + b0 + t]);
+            for (int t = 0; t < c; ++t) mac(g, sA[(b0 + t) * ld + i], opc<CJ>(sA[(b0 + c) * ld + b0 + t]));
             sG[c * nb + i] = g;
         }
         __syncthreads();
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 2) diag_ldl_kernel(const FrontDev* _
             for (int t = 0; t < kSub; ++t) {
                 const W g0 = sG[t * nb + ri], g1 = sG[t * nb + ri + 1];
                 const W l0 = opc<CJ>(sA[(b0 + t) * ld + cj]), l1 = opc<CJ>(sA[(b0 + t) * ld + cj + 1]);
-                a00 += g0 * l0; a01 += g0 * l1; a10 += g1 * l0; a11 += g1 * l1;
+                mac(a00, g0, l0); mac(a01, g0, l1); mac(a10, g1, l0); mac(a11, g1, l1);
             }
             sA[cj * ld + ri] -= a00;
             sA[cj * ld + ri + 1] -= a10;
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 2) diag_ldl_kernel(const FrontDev* _
                         // Linv[16 kk + t][16 j + c]; Linv_jj is unit lower triangular
                         const W lv = j < kk ? sA[(kSub * kk + t) * ld + kSub * j + c]
                                             : (t == c ? vone<W>() : (t > c ? sA[(kSub * kk + t) * ld + kSub * j + c] : W{}));
-                        acc[j] += lik * lv;
+                        mac(acc[j], lik, lv);
                     }
                 }
             }
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, 2) diag_ldl_kernel(const FrontDev* _
             for (int t = 0; t < r; ++t) {
                 const W lit = sA[R * ld + kSub * i + t];                            // Linv_ii[r][t]
 #pragma unroll
-                for (int j = 0; j < i; ++j) acc[j] += lit * sG[(j * kSub + c) * kSub + t];
+                for (int j = 0; j < i; ++j) mac(acc[j], lit, sG[(j * kSub + c) * kSub + t]);
             }
 #pragma unroll
             for (int j = 0; j < i; ++j) sA[R * ld + kSub * j + c] = W{} - acc[j];
