@@ -3,14 +3,20 @@
 // for one 128-row tile of the rows below a 64-wide diagonal block (the Trsm
 // of FrontLDL, include/clique/numeric/ldl/local_front.hpp:56-62).
 //
-// One CTA per tile, 192 threads:
-//   warps 0-3  thread = tile row: find the row's largest |Re|, |Im| over
-//              its 64 columns, write the row of A21 scaled by a power of two
-//              as FP16 hi / lo planes into shared memory; later the
-//              epilogue for the same row.
-//   warps 4-5  thread = column c of W: the same for row c of the B operand,
-//              B[c][t] = W[t][c] = U[t][c] / d_c; warp 4 lane 0 then issues
+// One CTA per tile, 384 threads, two to a row of either operand (one for its
+// first 32 columns, one for the others; the rows' maxima meet in shared memory):
+//   warps 0-7  tile rows: find the row's largest |Re|, |Im| over its 64
+//              columns, write the row of A21 scaled by a power of two as FP16
+//              hi / lo planes into shared memory; later the epilogue for the
+//              same half row.
+//   warps 8-11 columns c of W: the same for row c of the B operand,
+//              B[c][t] = W[t][c] = U[t][c] / d_c; warp 8 lane 0 then issues
 //              the tcgen05.mma kind::f16 (M = 128, N = 64, K = 16) products.
+// What bounds the launches of the large fronts (one or a few tiles a SM) is
+// the instruction stream of one row: the split of its entries and the packing
+// of the same entries for the update that follows: one thread to a row took
+// 25.1 us a launch on 40^3 complex fronts and 25.4 us on 101 x 99 x 90 real ones,
+// two take 17.6 and 21.1 us.
 // The 2xFP16 split and its accuracy are those of the update kernel
 // (tc_gemm2.cu): X = X_hi + X_lo after row scaling, three products per
 // real product.  The epilogue multiplies by the two inverse scales, writes
@@ -25,7 +31,9 @@ namespace cliqgpu {
 namespace tc2 {
 
 constexpr int kPanelRows = 128;
-constexpr int kPanelThreads = 192;
+constexpr int kPanelHalf = kTile / 2;             // columns per thread
+constexpr int kPanelAThreads = 2 * kPanelRows;
+constexpr int kPanelThreads = kPanelAThreads + 2 * kTile;
 constexpr int kPanelK = kTile;                    // 64 columns of the diagonal block
 constexpr int kPanelKS = 16;                      // k per kind::f16 MMA
 constexpr int kPanelSteps = kPanelK / kPanelKS;   // 4
@@ -121,12 +129,13 @@ __global__ void __launch_bounds__(kPanelThreads, 2) panel_tc_kernel(const FrontD
     // epilogue does not wait for them
     __shared__ int64_t s_pk[4];   // packA, packB, scaleA, scaleB (float offsets)
     __shared__ int32_t s_pkn[2];  // K, N
+    __shared__ float s_mx[2][2][kPanelRows + kTile];   // row maxima of the operands, then of L21 and S21, by half
     const bool prepack = probs && it.w >= 0;
     if (threadIdx.x == 0) {
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x == kPanelRows && prepack) {
+    if (threadIdx.x == kPanelAThreads && prepack) {
         const GemmProb& pr = probs[it.w];
         s_pk[0] = pr.packA; s_pk[1] = pr.packB; s_pk[2] = pr.scaleA; s_pk[3] = pr.scaleB;
         s_pkn[0] = pr.K; s_pkn[1] = pr.N;
@@ -135,54 +144,53 @@ __global__ void __launch_bounds__(kPanelThreads, 2) panel_tc_kernel(const FrontD
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)), "r"(PC::kTmem) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (threadIdx.x < kPanelRows) {
-        // ---- A: row i of A21, all 64 columns loaded at once into registers ----
-        const int i = threadIdx.x;
-        const bool vr = i < rows;
-        const int64_t a0 = f.L + r0 + i + (int64_t)k * f.m;
-        X v[nb];
+    // this thread's half row of an operand: row i of A21, or row c of W^T, B[c][t] = U[t][c] / d_c
+    const bool isA = threadIdx.x < kPanelAThreads;
+    const int row = isA ? threadIdx.x % kPanelRows : (threadIdx.x - kPanelAThreads) % kTile;
+    const int half = isA ? threadIdx.x / kPanelRows : (threadIdx.x - kPanelAThreads) / kTile;
+    const int t0 = kPanelHalf * half;
+    X v[kPanelHalf];
+    if (isA) {
+        const bool vr = row < rows;
+        const int64_t a0 = f.L + r0 + row + (int64_t)(k + t0) * f.m;
 #pragma unroll
-        for (int t = 0; t < nb; ++t) v[t] = (vr && t < kb) ? ldv<float, C>(L, a0 + (int64_t)t * f.m) : X{};
-        float mx = 0.f;
-#pragma unroll
-        for (int t = 0; t < nb; ++t) mx = fmaxf(mx, cmax(v[t]));
-        float inv;
-        const float s = row_scale(mx, &inv);
-        inv_a[i] = inv;
-#pragma unroll
-        for (int t = 0; t < nb; ++t) v[t] = v[t] * s;
-#pragma unroll
-        for (int ks = 0; ks < kPanelSteps; ++ks)
-            if (16 * ks < kb) put_row16<C>(sAop, i, ks, v + 16 * ks, kPanelSteps * PC::kABlock, PC::kABlock);
+        for (int t = 0; t < kPanelHalf; ++t) v[t] = (vr && t0 + t < kb) ? ldv<float, C>(L, a0 + (int64_t)t * f.m) : X{};
     } else {
-        // ---- B: row c of W^T, B[c][t] = U[t][c] / d_c ----
-        const int c = threadIdx.x - kPanelRows;
         const X* U = reinterpret_cast<const X*>(tinv) + (int64_t)slot * nb * nb;
-        X rd{};
-        if (c < kb) {
-            const W d = reinterpret_cast<const W*>(D)[f.off + k + c];
-            rd = conv<X>(W{} + vone<W>() / d);
-            s_d[c] = conv<X>(d);
-        } else {
-            s_d[c] = X{};
-        }
-        X v[nb];
 #pragma unroll
-        for (int t = 0; t < nb; ++t) v[t] = (t < kb && c < kb) ? U[t * nb + c] : X{};
+        for (int t = 0; t < kPanelHalf; ++t) v[t] = (t0 + t < kb && row < kb) ? U[(t0 + t) * nb + row] : X{};
+        X rd{};
+        if (row < kb) {
+            const W d = reinterpret_cast<const W*>(D)[f.off + k + row];
+            rd = conv<X>(W{} + vone<W>() / d);
+            if (half == 0) s_d[row] = conv<X>(d);
+        } else if (half == 0) {
+            s_d[row] = X{};
+        }
+#pragma unroll
+        for (int t = 0; t < kPanelHalf; ++t) v[t] = v[t] * rd;
+    }
+    {
         float mx = 0.f;
 #pragma unroll
-        for (int t = 0; t < nb; ++t) {
-            v[t] = v[t] * rd;
-            mx = fmaxf(mx, cmax(v[t]));
-        }
+        for (int t = 0; t < kPanelHalf; ++t) mx = fmaxf(mx, cmax(v[t]));
+        s_mx[0][half][isA ? row : kPanelRows + row] = mx;
+    }
+    __syncthreads();
+    {
+        const int at = isA ? row : kPanelRows + row;
         float inv;
-        const float s = row_scale(mx, &inv);
-        inv_b[c] = inv;
+        const float s = row_scale(fmaxf(s_mx[0][0][at], s_mx[0][1][at]), &inv);
+        if (half == 0) (isA ? inv_a : inv_b)[row] = inv;
 #pragma unroll
-        for (int t = 0; t < nb; ++t) v[t] = v[t] * s;
+        for (int t = 0; t < kPanelHalf; ++t) v[t] = v[t] * s;
 #pragma unroll
-        for (int ks = 0; ks < kPanelSteps; ++ks)
-            if (16 * ks < kb) put_row16<C>(sBop, c, ks, v + 16 * ks, kPanelSteps * PC::kBBlock, PC::kBBlock);
+        for (int q = 0; q < kPanelHalf / 16; ++q) {
+            const int ks = kPanelHalf / 16 * half + q;
+            if (16 * ks >= kb) break;
+            if (isA) put_row16<C>(sAop, row, ks, v + 16 * q, kPanelSteps * PC::kABlock, PC::kABlock);
+            else put_row16<C>(sBop, row, ks, v + 16 * q, kPanelSteps * PC::kBBlock, PC::kBBlock);
+        }
     }
     // operands written by the generic proxy, read by the tensor cores
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -191,7 +199,7 @@ __global__ void __launch_bounds__(kPanelThreads, 2) panel_tc_kernel(const FrontD
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (warp == 4) {
+    if (warp == kPanelAThreads / 32) {
         if (lane == 0) {
             const uint32_t idp = idesc_f16(kPanelRows, nb, false), idn = idesc_f16(kPanelRows, nb, true);
             const uint32_t dre = tmem, dim = tmem + nb;
@@ -219,19 +227,20 @@ __global__ void __launch_bounds__(kPanelThreads, 2) panel_tc_kernel(const FrontD
             mma_commit(done);
         }
         __syncwarp();
-    } else if (warp < 4) {
-        // ---- epilogue: thread = row i (TMEM lane i) ----
-        const bool ok = mbar_wait(done, 0, status, 6);
+    }
+    // ---- epilogue: thread = half of row i (TMEM lane i) ----
+    bool ok = false;
+    const int i = row;
+    const bool vr = i < rows;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp % 4) * 32) << 16);
+    if (isA) {
+        ok = mbar_wait(done, 0, status, 6);
         tc_fence_after();
+        float ml = 0.f, ms = 0.f;
         if (ok) {
-            const int i = warp * 32 + lane;
-            const bool vr = i < rows;
             const float ia = inv_a[i];
-            const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-            const int nT = (f.n + nb - 1) / nb;
-            float ml = 0.f, ms = 0.f;
 #pragma unroll 1
-            for (int c0 = 0; c0 < nb; c0 += 16) {
+            for (int c0 = t0; c0 < t0 + kPanelHalf; c0 += 16) {
                 float re[16], im[16];
                 tmem_ld16(lane_base + c0, re);
                 if constexpr (C) tmem_ld16(lane_base + nb + c0, im);
@@ -239,23 +248,33 @@ __global__ void __launch_bounds__(kPanelThreads, 2) panel_tc_kernel(const FrontD
                 for (int q = 0; q < 16; ++q) {
                     const int c = c0 + q;
                     const float sc = ia * inv_b[c];
-                    X v;
-                    if constexpr (C) v = X{re[q] * sc, im[q] * sc}; else v = re[q] * sc;
-                    if (c >= kb) v = X{};
+                    X x;
+                    if constexpr (C) x = X{re[q] * sc, im[q] * sc}; else x = re[q] * sc;
+                    if (c >= kb) x = X{};
                     if (vr && c < kb) {
-                        stv<float, C>(L, f.L + r0 + i + (int64_t)(k + c) * f.m, v);
-                        ml = fmaxf(ml, cmax(v));
-                        ms = fmaxf(ms, cmax(v * s_d[c]));
+                        stv<float, C>(L, f.L + r0 + i + (int64_t)(k + c) * f.m, x);
+                        ml = fmaxf(ml, cmax(x));
+                        ms = fmaxf(ms, cmax(x * s_d[c]));
                     }
                 }
             }
-            if (eblk && vr) {
-                const int64_t row = r0 + i;
-                const int64_t eb = f.eblk + row * nT + k / nb;
+        }
+        s_mx[0][half][i] = ml;   // (the operands' maxima were read before the last barrier)
+        s_mx[1][half][i] = ms;
+    }
+    __syncthreads();
+    if (isA && ok) {
+        {
+            const float ia = inv_a[i];
+            const float ml = fmaxf(s_mx[0][0][i], s_mx[0][1][i]), ms = fmaxf(s_mx[1][0][i], s_mx[1][1][i]);
+            const int nT = (f.n + nb - 1) / nb;
+            if (eblk && vr && half == 0) {
+                const int64_t row_g = r0 + i;
+                const int64_t eb = f.eblk + row_g * nT + k / nb;
                 eblk[eb] = __float_as_uint(ml);
                 eblk[eblk_total + eb] = __float_as_uint(ms);
-                atomicMax(&erow[f.erow + row], __float_as_uint(ml));
-                atomicMax(&erow[erow_total + f.erow + row], __float_as_uint(ms));
+                atomicMax(&erow[f.erow + row_g], __float_as_uint(ml));
+                atomicMax(&erow[erow_total + f.erow + row_g], __float_as_uint(ms));
             }
             // packed operands of the following in-panel update (rows of this
             // tile are rows tile*128 + i of its problem, K = kb): the A planes
@@ -278,10 +297,12 @@ __global__ void __launch_bounds__(kPanelThreads, 2) panel_tc_kernel(const FrontD
                 };
                 float inv_sa, inv_ss;
                 const float sa = scale_of(vr ? ml : 0.f, &inv_sa), ss = scale_of(vr && rp < pN ? ms : 0.f, &inv_ss);
-                pack[scaleA + rp] = inv_sa;
-                if (srow) pack[scaleB + rp] = inv_ss;
+                if (half == 0) {
+                    pack[scaleA + rp] = inv_sa;
+                    if (srow) pack[scaleB + rp] = inv_ss;
+                }
 #pragma unroll 1
-                for (int ks = 0; ks < nks; ++ks) {
+                for (int ks = kPanelHalf / 16 * half; ks < min(nks, kPanelHalf / 16 * (half + 1)); ++ks) {
                     float re[16], im[16];
                     tmem_ld16(lane_base + 16 * ks, re);
                     if constexpr (C) tmem_ld16(lane_base + nb + 16 * ks, im);
