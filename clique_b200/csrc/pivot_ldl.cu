@@ -174,57 +174,52 @@ __device__ __forceinline__ void block_argmax(T& v, int& idx, T* sv, int* si) {
 }
 
 // ---------------------------------------------------------------------------
-// LDL^T without interchanges of the kSpec x kSpec (w used) block of a group
-// of speculative columns, by one warp: lane r (and r + 16) holds row r.  The
-// rows' pending update is sum_p L(r, p) B(c, p) over the panel's np factored
-// columns, the two half-warps taking alternate p.  Leaves L11 (unit lower, column
-// by column), the pivots and their reciprocals, and returns the first column
-// whose pivot fails the Bunch-Kaufman test against the block's own rows (or
-// whose reciprocal would leave the range); w when none does.
+// LDL^T without interchanges of the kSpec x kSpec (w used) block s_a of a
+// group of speculative columns, by one warp: lanes r and r + 16 hold the even
+// and the odd columns of row r.  Leaves L11 (unit lower, column by column),
+// the pivots and their reciprocals, and returns the first column whose pivot
+// fails the Bunch-Kaufman test against the block's own rows (or whose
+// reciprocal would leave the range); w when none does.
 // ---------------------------------------------------------------------------
 template <class T, bool C, bool CJ>
-__device__ __forceinline__ int spec_block(int np, int w, const V<T, C>* s_l, const V<T, C>* s_b, const V<T, C>* s_a,
-                                          V<T, C>* s_l11, V<T, C>* s_dn, V<T, C>* s_rd) {
+__device__ __forceinline__ int spec_block(int w, const V<T, C>* s_a, V<T, C>* s_l11, V<T, C>* s_dn, V<T, C>* s_rd) {
     using X = V<T, C>;
     const int lane = threadIdx.x & 31, r = lane & (kSpec - 1), half = lane / kSpec;
-    X a[kSpec];
+    X a[kSpec / 2];   // column 2 t + half
 #pragma unroll
-    for (int c = 0; c < kSpec; ++c) a[c] = (half == 0 && r < w && c <= r) ? s_a[c * kSpec + r] : X{};
-    for (int p = half; p < np; p += 2) {
-        const X l = neg(s_l[p * kSpec + r]);
-#pragma unroll
-        for (int c = 0; c < kSpec; ++c) mac(a[c], l, s_b[p * kSpec + c]);
-    }
+    for (int t = 0; t < kSpec / 2; ++t) a[t] = s_a[(2 * t + half) * kSpec + r];
     auto shfl = [](X v, int src) -> X {
         if constexpr (C) return X{__shfl_sync(0xffffffffu, v.r, src), __shfl_sync(0xffffffffu, v.i, src)};
         else return __shfl_sync(0xffffffffu, v, src);
     };
-#pragma unroll
-    for (int c = 0; c < kSpec; ++c) a[c] += shfl(a[c], lane ^ kSpec);
     int fail = w;
 #pragma unroll
     for (int j = 0; j < kSpec; ++j) {
         if (j < w) {
-            X d = shfl(a[j], j);
+            const int owner = kSpec * (j & 1);   // the half that holds column j
+            const X aj = shfl(a[j / 2], owner + r);
+            X d = shfl(a[j / 2], owner + j);
             if constexpr (CJ) d = realpart(d);
             const T md = mag1(d);
             const bool zero = md == T(0);
             const T lo = sizeof(T) == 4 ? T(1e-30) : T(1e-290), hi = sizeof(T) == 4 ? T(1e30) : T(1e290);
-            const bool bad = r > j && r < w && !(md >= (T)kAlpha * mag1(a[j]));
+            const bool bad = r > j && r < w && !(md >= (T)kAlpha * mag1(aj));
             if (__ballot_sync(0xffffffffu, bad || !(zero || (md > lo && md < hi)))) fail = min(fail, j);
             X rd{};
-            if constexpr (CJ) rd.r = zero ? T(0) : T(1) / d.r;
+            if constexpr (CJ && sizeof(T) == 4) rd.r = zero ? T(0) : T(1) / d.r;
+            else if constexpr (CJ) rd.r = zero ? T(0) : pivot_recip(d.r);
             else rd = zero ? X{} : pivot_recip(d);
-            const X l = a[j] * rd;
+            const X l = aj * rd;
             if (lane == 0) {
                 s_dn[j] = d;
                 s_rd[j] = rd;
             }
             if (half == 0) s_l11[j * kSpec + r] = r > j ? l : X{};
+            const X nl = neg(l);
 #pragma unroll
-            for (int c = j + 1; c < kSpec; ++c) {
-                const X b = opc<CJ>(shfl(a[j], c));
-                mac(a[c], neg(l), b);   // (used for r >= c only)
+            for (int t = j / 2; t < kSpec / 2; ++t) {   // (entries of rows r >= 2 t + half are used)
+                const X b = opc<CJ>(shfl(a[j / 2], owner + min(2 * t + half, kSpec - 1)));
+                if (2 * t + half > j) mac(a[t], nl, b);
             }
         }
     }
@@ -243,18 +238,19 @@ __device__ __forceinline__ int spec_block(int np, int w, const V<T, C>* s_l, con
 // diagonal entry without an interchange, |a_kk| >= alpha max_i |a_ik|, in
 // every one of them: no interchange means that the columns are those of the
 // unpivoted elimination, so the group is eliminated without a search (its
-// diagonal block by one warp of every CTA, the rows below it one a thread,
-// with the group's kSpec entries in registers) and each row tests its own
+// diagonal block updated by every CTA and factored by one warp of it, the rows
+// below it one a thread, with the group's kSpec entries in registers) and each row tests its own
 // entries against the pivots.  The first column in which any row fails ends
 // the accepted prefix (the maximum over rows passes exactly when every row
 // does), nothing of the later columns has been written, and that column goes
 // through the general step below: candidate column and, where needed, row,
 // search, interchange, 1 x 1 or 2 x 2 pivot.  What bounds the general step is
 // its chain of L2 round trips and cluster barriers, 8.4 us a column with
-// 8 CTAs; a group of 16 columns passes two barriers.  Pivoted factor + refined
-// solve of 48^3 Helmholtz, CFP32: 56.3 -> 21.4 ms (panels were 41 ms of it);
-// indefinite operators, FP64: Hermitian 40 x 37 x 33 (1929 interchanged rows
-// in 48840) 28.4 -> 22.3 ms, real 29 x 27 x 23 in graph order 6.8 -> 5.2 ms.
+// 8 CTAs; a group of 16 columns passes two barriers.  Pivoted factor + solve,
+// column by column and now: 48^3 Helmholtz, CFP32 + refinement, 56.3 -> 17 ms
+// (panels 41 -> 6 ms); indefinite operators, FP64: Hermitian 40 x 37 x 33 (1929
+// interchanged rows in 48840) 28.5 -> 17.4 ms (panels 18.8 -> 10.6), real 29 x 27 x 23
+// in graph order 6.8 -> 4.2 ms.
 // ---------------------------------------------------------------------------
 template <class T, bool C, bool CJ, int G = 1>
 __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const FrontDev* __restrict__ F, const int32_t* __restrict__ fl,
@@ -336,8 +332,28 @@ __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const Fron
             }
             __syncthreads();
             const int i0 = k + w;
+            // this thread's first row, on its way while the block's pending update is applied
+            X y[kSpec];
+            {
+                const int i = i0 + rank * rt + tid;
+#pragma unroll
+                for (int c = 0; c < kSpec; ++c) y[c] = (tid < rt && i < n && c < w) ? ld(L, at(i, k + c)) : X{};
+            }
+            for (int idx = tid; idx < kSpec * kSpec; idx += nt) {
+                const int r = idx % kSpec, c = idx / kSpec;
+                if (c > r) continue;
+                X a0 = s_ga[idx], a1{};
+                int p = 0;
+                for (; p + 2 <= np; p += 2) {
+                    mac(a0, neg(s_gl[p * kSpec + r]), s_gb[p * kSpec + c]);
+                    mac(a1, neg(s_gl[(p + 1) * kSpec + r]), s_gb[(p + 1) * kSpec + c]);
+                }
+                if (p < np) mac(a0, neg(s_gl[p * kSpec + r]), s_gb[p * kSpec + c]);
+                s_ga[idx] = a0 + a1;
+            }
+            __syncthreads();
             if (tid >= rt) {   // the last warp
-                const int f0 = spec_block<T, C, CJ>(np, w, s_gl, s_gb, s_ga, s_gl11, s_gd, s_grd);
+                const int f0 = spec_block<T, C, CJ>(w, s_ga, s_gl11, s_gd, s_grd);
                 if (tid == rt) atomicMin(&s_fail, f0);
                 __syncthreads();
             } else {
@@ -345,9 +361,10 @@ __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const Fron
                 for (int q = 0; q == 0 || q * rt < slots; ++q) {
                     const int i = i0 + rank * rt + tid + q * G * rt;
                     const bool in = i < n;
-                    X y[kSpec];
+                    if (q > 0) {
 #pragma unroll
-                    for (int c = 0; c < kSpec; ++c) y[c] = (in && c < w) ? ld(L, at(i, k + c)) : X{};
+                        for (int c = 0; c < kSpec; ++c) y[c] = (in && c < w) ? ld(L, at(i, k + c)) : X{};
+                    }
                     if (in) {
                         constexpr int kFly = C && sizeof(T) == 8 ? 4 : 8;   // loads in flight
                         int p = 0;
@@ -604,7 +621,9 @@ __global__ void __launch_bounds__(panel_threads<T>()) bk_panel_kernel(const Fron
 // shared memory (asynchronous copies, beside the loads of L11), then
 // substituted kSpec columns at a time with the group's entries in registers:
 // one entry of y = L21 D read back feeds kSpec products.  What bounds a
-// launch is that chain for one row.  For the 2xFP16 split of the Schur
+// launch is that chain for one row (48^3 CFP32: 85 us a launch with one product
+// per entry read back, 31 us so; 64-row CTAs on levels of few fronts took
+// longer, 61 against 43 us on real FP64: the loads of L11 have half the threads).  For the 2xFP16 split of the Schur
 // complements the row's largest |component| of L21 and of y (which |B| is)
 // goes into the two halves of erow (float bits), panel after panel.
 // ---------------------------------------------------------------------------
@@ -641,11 +660,11 @@ __global__ void __launch_bounds__(kLowerRows) bk_lower_kernel(const FrontDev* __
     for (int q = threadIdx.x; q < kb; q += kLowerRows) {
         s_d[q] = conv<X>(reinterpret_cast<const W*>(D)[f.off + j0 + q]);
         s_e[q] = conv<X>(reinterpret_cast<const W*>(E)[f.off + j0 + q]);
-        // complex symmetric: reciprocals of the 1 x 1 pivots (a complex division
-        // is a few real ones in a row); 0 leaves an entry to the division (real
-        // pivots, pivots near the ends of the range)
+        // reciprocals of the 1 x 1 pivots where a division is several operations
+        // in a row (FP64, complex symmetric); 0 leaves an entry to the division
+        // (real FP32 pivots, pivots near the ends of the range)
         const T md = mag1(s_d[q]);
-        const bool ok = C && !CJ && md > (sizeof(T) == 4 ? T(1e-30) : T(1e-290)) && md < (sizeof(T) == 4 ? T(1e30) : T(1e290));
+        const bool ok = (sizeof(T) == 8 || (C && !CJ)) && md > (sizeof(T) == 4 ? T(1e-30) : T(1e-290)) && md < (sizeof(T) == 4 ? T(1e30) : T(1e290));
         s_rd[q] = ok ? pivot_recip(s_d[q]) : X{};
     }
     __pipeline_wait_prior(0);   // (a thread reads back only the row it fetched)
@@ -692,7 +711,7 @@ __global__ void __launch_bounds__(kLowerRows) bk_lower_kernel(const FrontDev* __
             const X d11 = s_d[q - 1], e = s_e[q - 1];
             l = (y0 * d11 - y[(q - 1) * kLowerRows] * opc<CJ>(e)) / (d11 * d - e * opc<CJ>(e));
         } else {
-            if constexpr (CJ) l = d.r == T(0) ? X{} : X{y0.r / d.r, y0.i / d.r};
+            if constexpr (CJ) l = !is_zero(rd) ? y0 * rd.r : d.r == T(0) ? X{} : X{y0.r / d.r, y0.i / d.r};
             else l = !is_zero(rd) ? y0 * rd : is_zero(d) ? X{} : y0 / d;
         }
         ml = fmaxf(ml, big(l));
