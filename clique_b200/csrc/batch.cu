@@ -165,8 +165,8 @@ static int batch_issue(Plan& P, const double* values, const double* B, double* X
     if ((st = run_factor_dispatch(P)) != CLIQ_OK) return st;
     // sweep flags: the epochs of a replayed graph repeat, so clear what an
     // earlier replay published
-    cudaMemsetAsync(P.flags, 0, sizeof(int32_t) * (size_t)(P.flags_total + P.helpers_total), P.stream);
-    cudaMemsetAsync(P.xprog, 0, sizeof(unsigned long long) * (size_t)std::max(P.num_fronts, 1), P.stream);
+    cudaMemsetAsync(P.flags, 0, sizeof(int32_t) * kSweepSets * (size_t)(P.flags_total + P.helpers_total), P.stream);
+    cudaMemsetAsync(P.xprog, 0, sizeof(unsigned long long) * kSweepSets * (size_t)std::max(P.num_fronts, 1), P.stream);
     if (cudaMemcpy2DAsync(b, colbytes, B, sizeof(double) * w * (size_t)ld, colbytes, nrhs, cudaMemcpyDeviceToDevice,
                           P.stream) != cudaSuccess)
         return check_cuda("batch: B");

@@ -59,6 +59,12 @@ constexpr int kEAGroups = 4;     // columns swept at a time on levels of short f
 // product of that inverse with the coupling tile.
 constexpr int kSolveLag = 2;
 constexpr int kSolveRhsChunk = 16;   // right-hand sides per sweep (partial-sum stride)
+// complex FP64 sweeps (8 right-hand sides at a time) of levels of few large
+// fronts run four right-hand sides to a CTA, the groups side by side with
+// flags of their own (kSweepSets of them)
+constexpr int kSweepCols = 4;
+constexpr int kSweepSets = 2;
+constexpr int kSplitFronts = 8;      // most fronts of such a level
 constexpr int kGatherRows = 256;     // front rows per gather CTA (grid y of the gather launch)
 constexpr int kLowerChunkTiles = 16; // backward: 64-row tiles below the pivots per helper
 // sweep work items {front, kind, block, chunk}

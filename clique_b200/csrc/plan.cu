@@ -752,14 +752,14 @@ int build_plan(Plan& P, const cliq_symm_info* info, int64_t n, const int32_t* ma
     TRY(dev_upload(P, &P.dest, dest));
     TRY(dev_upload(P, &P.perm, inv));
     TRY(dev_upload(P, &P.level_fronts, level_fronts));
-    std::vector<int32_t> zeros_flags(P.flags_total + P.helpers_total, 0);
+    std::vector<int32_t> zeros_flags(kSweepSets * (size_t)(P.flags_total + P.helpers_total), 0);
     TRY(dev_upload(P, &P.flags, zeros_flags));
     P.nchain_items = (int32_t)(chain_items.size() / 4);
     if (chain_items.empty()) chain_items.assign(4, 0);
     TRY(dev_upload(P, &P.chain_items, chain_items));
-    std::vector<unsigned long long> zprog(std::max(nn, 1), 0ull);
+    std::vector<unsigned long long> zprog(kSweepSets * (size_t)std::max(nn, 1), 0ull);
     TRY(dev_upload(P, &P.xprog, zprog));
-    std::vector<int32_t> zt(2 * (P.max_depth + 1) + 2, 0);
+    std::vector<int32_t> zt(kSweepSets * (2 * (P.max_depth + 1) + 2), 0);
     TRY(dev_upload(P, &P.tickets, zt));
     std::vector<int32_t> st = {INT_MAX, 0, 0, 0};
     TRY(dev_upload(P, &P.status, st));

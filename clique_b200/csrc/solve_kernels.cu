@@ -559,12 +559,18 @@ struct SweepArgs {
     void* w0;
     void* w1;
     const int32_t* lower;
-    int nrhs;
+    int nrhs;               // of this CTA's group of columns
+    int wrhs, jcol;         // right-hand sides of the W layout, first column of the group
     int32_t* status;
     // 1: substitution form of the chain steps, x_s = L_ss^{-1} (t_s - L_{s,s-1} x_{s-1})
     // (and its backward counterpart) with the workers publishing t_s; 0: the
     // product form x_s = y_s - M_s x_{s-1} through the stored chain tiles
     int exact;
+};
+
+// one set of arguments per group of columns (grid y)
+struct SweepSets {
+    SweepArgs a[kSweepSets];
 };
 
 // Forward chain of front fi: x_s = y_s - M_s x_{s-1}.  Step s multiplies the
@@ -746,7 +752,7 @@ __device__ void fwd_whole(const SweepArgs& a, const FrontDev& f, int nT, int r, 
 #pragma unroll
         for (int b = 0; b < NR / kQ; ++b) {
             const int j = q + kQ * b;
-            wv[b] = (r < nr && j < a.nrhs) ? ldv<T, C>(wb, f.W * a.nrhs + (R0 - f.n + r) + (int64_t)j * f.u) : Xv{};
+            wv[b] = (r < nr && j < a.nrhs) ? ldv<T, C>(wb, f.W * a.wrhs + (R0 - f.n + r) + (int64_t)(j + a.jcol) * f.u) : Xv{};
         }
     };
     auto unit = [&](int u, const Xv (&cur)[kE], Xv (&oth)[kE]) {
@@ -760,7 +766,7 @@ __device__ void fwd_whole(const SweepArgs& a, const FrontDev& f, int nT, int r, 
 #pragma unroll
             for (int b = 0; b < NR / kQ; ++b) {
                 const int j = q + kQ * b;
-                if (r < nr && j < a.nrhs) stv<T, C>(wb, f.W * a.nrhs + (R0 - f.n + r) + (int64_t)j * f.u, wv[b] - out[b]);
+                if (r < nr && j < a.nrhs) stv<T, C>(wb, f.W * a.wrhs + (R0 - f.n + r) + (int64_t)(j + a.jcol) * f.u, wv[b] - out[b]);
             }
             if (i + 1 < ntl) load_w(i + 1);
 #pragma unroll
@@ -894,7 +900,7 @@ __device__ void fwd_worker(const SweepArgs& a, const FrontDev& f, int fi, int nT
         for (int b = 0; b < NR / kQ; ++b) {
             const int j = q + kQ * b;
             if (j < a.nrhs) {
-                const int64_t e = f.W * a.nrhs + (R0 - f.n + r) + (int64_t)j * f.u;
+                const int64_t e = f.W * a.wrhs + (R0 - f.n + r) + (int64_t)(j + a.jcol) * f.u;
                 stv<T, C>(wb, e, ldv<T, C>(wb, e) - out[b]);
             }
         }
@@ -902,7 +908,8 @@ __device__ void fwd_worker(const SweepArgs& a, const FrontDev& f, int fi, int nT
 }
 
 template <class T, bool C, int NR>
-__global__ void __launch_bounds__(kSolveThreads, sweep_min_blocks<T, C, NR>()) fwd_sweep_kernel(SweepArgs a) {
+__global__ void __launch_bounds__(kSolveThreads, sweep_min_blocks<T, C, NR>()) fwd_sweep_kernel(const __grid_constant__ SweepSets sets) {
+    const SweepArgs& a = sets.a[blockIdx.y];
     using Xv = V<T, C>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Xv* sx = reinterpret_cast<Xv*>(smem_raw);     // 2 x [64][NR]
@@ -1319,7 +1326,8 @@ __device__ void bwd_worker(const SweepArgs& a, const FrontDev& f, int fi, int nT
 }
 
 template <class T, bool C, bool CJ, int NR>
-__global__ void __launch_bounds__(kSolveThreads, sweep_min_blocks<T, C, NR>()) bwd_sweep_kernel(SweepArgs a) {
+__global__ void __launch_bounds__(kSolveThreads, sweep_min_blocks<T, C, NR>()) bwd_sweep_kernel(const __grid_constant__ SweepSets sets) {
+    const SweepArgs& a = sets.a[blockIdx.y];
     using Xv = V<T, C>;
     constexpr int ldl = kTile + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1350,42 +1358,72 @@ template <class T, bool C, bool CJ, int NR>
 static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
     using Xv = V<T, C>;
     const size_t smem_fwd = sizeof(Xv) * (4 + kQ) * kTile * NR;
-    const size_t smem_bwd = sizeof(Xv) * ((3 + kQ) * kTile * NR + kTile * (kTile + 1)) + sizeof(int32_t) * kLowerChunkTiles * kTile;
+    auto bwd_smem = [](int cols) {
+        return sizeof(Xv) * ((3 + kQ) * kTile * cols + kTile * (kTile + 1)) + sizeof(int32_t) * kLowerChunkTiles * kTile;
+    };
     constexpr size_t smem_tiny = tiny_smem_bytes<T, C, NR>();
     static bool attr_done = false;
     if (!attr_done) {
         cudaFuncSetAttribute(fwd_sweep_kernel<T, C, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fwd);
-        cudaFuncSetAttribute(bwd_sweep_kernel<T, C, CJ, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bwd);
+        cudaFuncSetAttribute(bwd_sweep_kernel<T, C, CJ, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem(NR));
+        if (C && sizeof(T) == 8 && NR > kSweepCols) {   // levels swept in groups of columns
+            cudaFuncSetAttribute(fwd_sweep_kernel<T, C, kSweepCols>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(smem_fwd / NR * kSweepCols));
+            cudaFuncSetAttribute(bwd_sweep_kernel<T, C, CJ, kSweepCols>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bwd_smem(kSweepCols));
+        }
         cudaFuncSetAttribute(tiny_fwd_kernel<T, C, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_tiny);
         cudaFuncSetAttribute(tiny_bwd_kernel<T, C, CJ, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_tiny);
         attr_done = true;
     }
     const int4* items = reinterpret_cast<const int4*>(P.items);
-    SweepArgs a{};
-    a.F = P.fronts;
-    a.xprog = P.xprog;
-    a.pflags = P.flags;
-    a.L = P.L;
-    a.dinv = P.dinv;
-    a.dinvT = P.dinvT;
-    a.m1 = P.m1;
-    a.n1 = P.n1;
-    a.partial = P.partial;
-    a.hpart = P.hpart;
-    a.hflags = P.flags + P.flags_total;
-    a.X = X;
-    a.ldx = P.n;
-    a.w0 = P.wpool[0];
-    a.w1 = P.wpool[1];
-    a.lower = P.lower;
-    a.nrhs = nrhs;
-    a.status = P.status;
-    a.exact = P.solve_exact;
+    const int nlev = P.max_depth + 1;
+    // the sweep of one level over groups of `cols` columns side by side
+    auto sets_of = [&](int cols, const int4* lv_items, int ticket) {
+        SweepSets sets{};
+        for (int y = 0; y < kSweepSets && y * cols < nrhs; ++y) {
+            SweepArgs& a = sets.a[y];
+            const int64_t col0 = (int64_t)(C ? 2 : 1) * y * cols;   // in scalars
+            a.F = P.fronts;
+            a.items = lv_items;
+            a.ticket = P.tickets + (int64_t)y * 2 * nlev + ticket;
+            a.xprog = P.xprog + (int64_t)y * P.num_fronts;
+            a.pflags = P.flags + (int64_t)y * (P.flags_total + P.helpers_total);
+            a.hflags = a.pflags + P.flags_total;
+            a.epoch = P.epoch;
+            a.L = P.L;
+            a.dinv = P.dinv;
+            a.dinvT = P.dinvT;
+            a.m1 = P.m1;
+            a.n1 = P.n1;
+            a.partial = reinterpret_cast<T*>(P.partial) + col0 * kTile;
+            a.hpart = reinterpret_cast<T*>(P.hpart) + col0 * kTile;
+            a.X = X + col0 * P.n;
+            a.ldx = P.n;
+            a.w0 = P.wpool[0];
+            a.w1 = P.wpool[1];
+            a.lower = P.lower;
+            a.nrhs = std::min(cols, nrhs - y * cols);
+            a.wrhs = nrhs;
+            a.jcol = y * cols;
+            a.status = P.status;
+            a.exact = P.solve_exact;
+        }
+        return sets;
+    };
+    // levels of few fronts wait for their chains, and a complex FP64 step takes
+    // as long as its products over the right-hand sides: groups of kSweepCols
+    // columns side by side (the five top levels of 56^3 with 8 columns: forward
+    // 910 -> 793 us, backward 1224 -> 957 us; real FP32 steps are not bound by
+    // their products, 16 columns in four groups took 618 us a level against 395)
+    constexpr bool kCanSplit = C && sizeof(T) == 8 && NR > kSweepCols;
+    static_assert(!kCanSplit || NR <= kSweepCols * kSweepSets, "a set of flags per group");
+    auto split = [&](const SolveLevel& lv) { return kCanSplit && lv.nfronts <= kSplitFronts; };
+    const unsigned groups = (unsigned)((nrhs + kSweepCols - 1) / kSweepCols);
     T* w0 = reinterpret_cast<T*>(P.wpool[0]);
     T* w1 = reinterpret_cast<T*>(P.wpool[1]);
-    const int nlev = P.max_depth + 1;
     int64_t launches = 0;
-    cudaMemsetAsync(P.tickets, 0, sizeof(int32_t) * 2 * nlev, P.stream);
+    cudaMemsetAsync(P.tickets, 0, sizeof(int32_t) * kSweepSets * 2 * nlev, P.stream);
     for (int d = P.max_depth; d >= 0; --d) {
         const SolveLevel& lv = P.solve_levels[d];
         if (lv.nfronts == 0) continue;
@@ -1402,10 +1440,12 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
             ++launches;
         }
         if (lv.nfwd > 0) {
-            a.items = items + lv.fwd_items;
-            a.ticket = P.tickets + 2 * d;
-            a.epoch = ++P.epoch;
-            fwd_sweep_kernel<T, C, NR><<<lv.nfwd, kSolveThreads, smem_fwd, P.stream>>>(a);
+            ++P.epoch;
+            if (split(lv))
+                fwd_sweep_kernel<T, C, kSweepCols><<<dim3(lv.nfwd, groups), kSolveThreads, smem_fwd / NR * kSweepCols, P.stream>>>(
+                    sets_of(kSweepCols, items + lv.fwd_items, 2 * d));
+            else
+                fwd_sweep_kernel<T, C, NR><<<lv.nfwd, kSolveThreads, smem_fwd, P.stream>>>(sets_of(NR, items + lv.fwd_items, 2 * d));
             ++launches;
         }
     }
@@ -1421,10 +1461,13 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
             ++launches;
         }
         if (lv.nbwd == 0) continue;
-        a.items = items + lv.bwd_items;
-        a.ticket = P.tickets + 2 * d + 1;
-        a.epoch = ++P.epoch;
-        bwd_sweep_kernel<T, C, CJ, NR><<<lv.nbwd, kSolveThreads, smem_bwd, P.stream>>>(a);
+        ++P.epoch;
+        if (split(lv))
+            bwd_sweep_kernel<T, C, CJ, kSweepCols><<<dim3(lv.nbwd, groups), kSolveThreads, bwd_smem(kSweepCols), P.stream>>>(
+                sets_of(kSweepCols, items + lv.bwd_items, 2 * d + 1));
+        else
+            bwd_sweep_kernel<T, C, CJ, NR><<<lv.nbwd, kSolveThreads, bwd_smem(NR), P.stream>>>(
+                sets_of(NR, items + lv.bwd_items, 2 * d + 1));
         ++launches;
     }
     return launches;

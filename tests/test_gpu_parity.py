@@ -730,3 +730,68 @@ def test_tiny_front_sizes(oracle, kind, nrhs, dims, cutoff):
     F = oracle.Fronts(S, A.values, is_complex=kind == "complex")
     assert F.ldl(96) == 0
     assert rel(X, F.solve(B.copy(order="F"))) <= 1e-10
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("half,width", [(72, 7), (31, 16), (18, 27), (60, 40)])
+def test_extend_add_item_shapes(oracle, kind, half, width):
+    """Two leaves of half x width pivots under a separator of width: leaf fronts
+    of 511, 512, 513 and 2440 rows (one or four columns swept at a time, one or
+    two row chunks), levels of few items.  The oracle's solution to 1e-10."""
+    dims = (2 * half + 1, width, 1)
+    A = ops.laplacian_3d(*dims, 4.2) if kind == "real" else ops.helmholtz_pml_3d(*dims, omega=9.0, b=2)
+    cutoff = half * width
+    _, info, L = build(A, dims, cutoff)
+    assert sorted(nd.size + len(nd.lowerStruct) for nd in info.localNodes) == [width] + 2 * [(half + 1) * width]
+    B = ops.random_rhs(A.n, 2, seed=3, complex_=kind == "complex")
+    X = cliq.Solve(info, L, B.copy(order="F"))
+    S = oracle.Symbolic(*dims, A.rowptr, A.colind, cutoff=cutoff)
+    F = oracle.Fronts(S, A.values, is_complex=kind == "complex")
+    assert F.ldl(96) == 0
+    assert rel(X, F.solve(B.copy(order="F"))) <= 1e-10
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("half,width", [(5, 13), (8, 12), (11, 9), (11, 16), (9, 19), (190, 1), (192, 1)])
+def test_fp32_panel_tiles(kind, half, width):
+    """FP32 leaves of half x width pivots over a separator of width rows: last
+    blocks of 1, 32, 35 and 48 columns, 126 to 129 rows below a block.  Against
+    the FP64 fronts: entries of L (at most 1) are sums of up to n products of
+    operands split to 22 bits, n * 3 * 2^-22 <= 2e-4 for n <= 258."""
+    dims, cutoff = (2 * half + 1, width, 1), half * width
+    csr = ops.laplacian_3d(*dims, 4.5)
+    if kind == "complex":
+        vals = csr.values.astype(np.complex128)
+        rows = np.repeat(np.arange(csr.n), np.diff(csr.rowptr))
+        vals[csr.colind == rows] *= 1 + 0.3j
+        csr = ops.CSR(csr.n, csr.rowptr, csr.colind, vals)
+    _, info, L64 = build(csr, dims, cutoff)
+    _, _, L32 = build(csr, dims, cutoff, precision="single")
+    for s in range(info.num_nodes):
+        (a, da), (b, db) = L64.front(s), L32.front(s)
+        assert np.abs(a - b).max() <= 2e-4
+        assert np.abs(da - db).max() <= 2e-4 * np.abs(da).max()
+
+
+@pytest.mark.parametrize("conjugate", [False, True])
+@pytest.mark.parametrize("nrhs", [4, 5, 8, 13])
+def test_complex_fp64_column_groups(oracle, conjugate, nrhs):
+    """Chains of 1 to 4 blocks swept in one or two groups of columns (complex
+    FP64, 8 columns at a time): the oracle's solution to 1e-10."""
+    dims, cutoff = (16, 15, 14), 80
+    if conjugate:
+        A = ops.laplacian_3d(*dims, 6.5)
+        vals = A.values.astype(np.complex128)
+        rows = np.repeat(np.arange(A.n), np.diff(A.rowptr))
+        off = A.colind != rows
+        vals[off] = vals[off] * np.exp(1j * 0.3 * np.sign(A.colind - rows))[off]
+        A = ops.CSR(A.n, A.rowptr, A.colind, vals)
+    else:
+        A = ops.helmholtz_pml_3d(*dims, omega=9.0, b=2)
+    _, info, L = build(A, dims, cutoff, conjugate=conjugate)
+    B = ops.random_rhs(A.n, nrhs, seed=nrhs, complex_=True)
+    X = cliq.Solve(info, L, B.copy(order="F"))
+    S = oracle.Symbolic(*dims, A.rowptr, A.colind, cutoff=cutoff)
+    F = oracle.Fronts(S, A.values, is_complex=True, conjugate=conjugate)
+    assert F.ldl(96) == 0
+    assert rel(X, F.solve(B.copy(order="F"))) <= 1e-10
