@@ -406,16 +406,21 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(const FrontDev* __restr
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) acc[a][b] = X{};
-    for (int t = 0; t < kb; ++t) {
-        X av[4], uv[4];
+    // U is upper triangular: rows 16 tb .. reach only the columns from 16 tb on
+    // (64^3 complex FP64: 46.5 -> 38.3 us a launch, the products bound it; real 11.9 -> 11.4)
 #pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = sA[(ty + 16 * a) * ldA + t];
+    for (int tb = 0; tb < 4; ++tb) {
+        for (int t = 16 * tb; t < min(kb, 16 * tb + 16); ++t) {
+            X av[4], uv[4];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) uv[b] = sU[t * nb + tx + 16 * b];
+            for (int a = 0; a < 4; ++a) av[a] = sA[(ty + 16 * a) * ldA + t];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+            for (int b = tb; b < 4; ++b) uv[b] = sU[t * nb + tx + 16 * b];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) mac(acc[a][b], av[a], uv[b]);
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = tb; b < 4; ++b) mac(acc[a][b], av[a], uv[b]);
+        }
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
