@@ -907,9 +907,11 @@ __device__ void fwd_worker(const SweepArgs& a, const FrontDev& f, int fi, int nT
     }
 }
 
-template <class T, bool C, int NR>
+// SPLIT: grid y selects the group of columns (a kernel of its own: arguments
+// read through an index made the other sweeps 3 to 8 % slower)
+template <class T, bool C, int NR, bool SPLIT = false>
 __global__ void __launch_bounds__(kSolveThreads, sweep_min_blocks<T, C, NR>()) fwd_sweep_kernel(const __grid_constant__ SweepSets sets) {
-    const SweepArgs& a = sets.a[blockIdx.y];
+    const SweepArgs& a = sets.a[SPLIT ? blockIdx.y : 0];
     using Xv = V<T, C>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Xv* sx = reinterpret_cast<Xv*>(smem_raw);     // 2 x [64][NR]
@@ -1325,9 +1327,9 @@ __device__ void bwd_worker(const SweepArgs& a, const FrontDev& f, int fi, int nT
     publish_flag(&a.pflags[f.flag_base + c], a.epoch);
 }
 
-template <class T, bool C, bool CJ, int NR>
+template <class T, bool C, bool CJ, int NR, bool SPLIT = false>
 __global__ void __launch_bounds__(kSolveThreads, sweep_min_blocks<T, C, NR>()) bwd_sweep_kernel(const __grid_constant__ SweepSets sets) {
-    const SweepArgs& a = sets.a[blockIdx.y];
+    const SweepArgs& a = sets.a[SPLIT ? blockIdx.y : 0];
     using Xv = V<T, C>;
     constexpr int ldl = kTile + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1366,10 +1368,10 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
     if (!attr_done) {
         cudaFuncSetAttribute(fwd_sweep_kernel<T, C, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fwd);
         cudaFuncSetAttribute(bwd_sweep_kernel<T, C, CJ, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem(NR));
-        if (C && sizeof(T) == 8 && NR > kSweepCols) {   // levels swept in groups of columns
-            cudaFuncSetAttribute(fwd_sweep_kernel<T, C, kSweepCols>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if constexpr (C && sizeof(T) == 8 && NR > kSweepCols) {   // levels swept in groups of columns
+            cudaFuncSetAttribute(fwd_sweep_kernel<T, C, kSweepCols, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(smem_fwd / NR * kSweepCols));
-            cudaFuncSetAttribute(bwd_sweep_kernel<T, C, CJ, kSweepCols>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(bwd_sweep_kernel<T, C, CJ, kSweepCols, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)bwd_smem(kSweepCols));
         }
         cudaFuncSetAttribute(tiny_fwd_kernel<T, C, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_tiny);
@@ -1418,8 +1420,7 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
     // their products, 16 columns in four groups took 618 us a level against 395)
     constexpr bool kCanSplit = C && sizeof(T) == 8 && NR > kSweepCols;
     static_assert(!kCanSplit || NR <= kSweepCols * kSweepSets, "a set of flags per group");
-    auto split = [&](const SolveLevel& lv) { return kCanSplit && lv.nfronts <= kSplitFronts; };
-    const unsigned groups = (unsigned)((nrhs + kSweepCols - 1) / kSweepCols);
+    [[maybe_unused]] const unsigned groups = (unsigned)((nrhs + kSweepCols - 1) / kSweepCols);
     T* w0 = reinterpret_cast<T*>(P.wpool[0]);
     T* w1 = reinterpret_cast<T*>(P.wpool[1]);
     int64_t launches = 0;
@@ -1441,10 +1442,15 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
         }
         if (lv.nfwd > 0) {
             ++P.epoch;
-            if (split(lv))
-                fwd_sweep_kernel<T, C, kSweepCols><<<dim3(lv.nfwd, groups), kSolveThreads, smem_fwd / NR * kSweepCols, P.stream>>>(
-                    sets_of(kSweepCols, items + lv.fwd_items, 2 * d));
-            else
+            bool done = false;
+            if constexpr (kCanSplit) {
+                if (lv.nfronts <= kSplitFronts) {
+                    fwd_sweep_kernel<T, C, kSweepCols, true><<<dim3(lv.nfwd, groups), kSolveThreads, smem_fwd / NR * kSweepCols,
+                                                               P.stream>>>(sets_of(kSweepCols, items + lv.fwd_items, 2 * d));
+                    done = true;
+                }
+            }
+            if (!done)
                 fwd_sweep_kernel<T, C, NR><<<lv.nfwd, kSolveThreads, smem_fwd, P.stream>>>(sets_of(NR, items + lv.fwd_items, 2 * d));
             ++launches;
         }
@@ -1462,10 +1468,15 @@ static int64_t run_sweeps(Plan& P, T* X, int nrhs) {
         }
         if (lv.nbwd == 0) continue;
         ++P.epoch;
-        if (split(lv))
-            bwd_sweep_kernel<T, C, CJ, kSweepCols><<<dim3(lv.nbwd, groups), kSolveThreads, bwd_smem(kSweepCols), P.stream>>>(
-                sets_of(kSweepCols, items + lv.bwd_items, 2 * d + 1));
-        else
+        bool done = false;
+        if constexpr (kCanSplit) {
+            if (lv.nfronts <= kSplitFronts) {
+                bwd_sweep_kernel<T, C, CJ, kSweepCols, true><<<dim3(lv.nbwd, groups), kSolveThreads, bwd_smem(kSweepCols), P.stream>>>(
+                    sets_of(kSweepCols, items + lv.bwd_items, 2 * d + 1));
+                done = true;
+            }
+        }
+        if (!done)
             bwd_sweep_kernel<T, C, CJ, NR><<<lv.nbwd, kSolveThreads, bwd_smem(NR), P.stream>>>(
                 sets_of(NR, items + lv.bwd_items, 2 * d + 1));
         ++launches;
